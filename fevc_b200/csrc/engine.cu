@@ -984,23 +984,15 @@ __global__ void k_center(uint32_t n, const double* __restrict__ b, const double*
 }
 
 // rz = sum of the per-block partials [blocks][K]; the count of active columns.
-// One block of SET_RZ_THREADS threads, blockDim / K lanes per column.
-constexpr int SET_RZ_THREADS = 1024;
 template <int K>
-__global__ void k_set_rz(const double* __restrict__ partial, int blocks, PcgState s) {
-  __shared__ double sm[SET_RZ_THREADS];
+__global__ void __launch_bounds__(STEP_THREADS) k_set_rz(const double* __restrict__ partial, int blocks, PcgState s) {
+  __shared__ double sum[K], scratch[STEP_THREADS];
   __shared__ int cnt;
   if (threadIdx.x == 0) cnt = 0;
-  const int groups = blockDim.x / K, o = threadIdx.x % K, g = threadIdx.x / K;
-  double acc = 0.0;
-  if (g < groups)
-    for (int b = g; b < blocks; b += groups) acc += partial[size_t(b) * K + o];
-  sm[threadIdx.x] = acc;
-  __syncthreads();
-  if (g == 0) {
-    double sum = 0.0;
-    for (int k = 0; k < groups; ++k) sum += sm[k * K + o];
-    s.rz[o] = sum;
+  redundant_finish<1, K>(partial, blocks, sum, scratch);
+  const int o = threadIdx.x;
+  if (o < K) {
+    s.rz[o] = sum[o];
     if (s.active[o]) atomicAdd(&cnt, 1);
   }
   __syncthreads();
@@ -1090,7 +1082,7 @@ void pcg_restart(DeviceEngine& e, BlockWork& w, Launch L, bool fresh, bool direc
   } else {
     k_jacobi_start<K><<<L.grid, THREADS, 0, L.s>>>(e.n, e.L_dinv.p, w.r.p, w.p.p, e.partial.p);
   }
-  k_set_rz<K><<<1, SET_RZ_THREADS, 0, L.s>>>(e.partial.p, L.grid, w.s);
+  k_set_rz<K><<<1, STEP_THREADS, 0, L.s>>>(e.partial.p, L.grid, w.s);
   CK_LAUNCH();
 }
 
@@ -1305,12 +1297,15 @@ template <int K>
 void mg_iteration(DeviceEngine& e, BlockWork& w, Launch L, cudaStream_t s) {
   double* pa = e.partial.p;
   double* pb = e.partial.p + size_t(L.grid) * K;
-  k_spmm_dot<K><<<L.grid, THREADS, 0, s>>>(e.n, e.L_ptr.p, e.L_col.p, e.L_val.p, e.L_diag.p, w.p.p, w.q.p, pa);
-  k_step_alpha<K><<<1, 128, 0, s>>>(pa, L.grid, w.s);
+  k_spmm_segments<K><<<L.grid, THREADS, 0, s>>>(e.lap_seg.count, e.lap_seg.ord_id.p, e.lap_seg.ord_begin.p,
+                                                e.lap_seg.ord_end.p, e.L_col.p, e.L_val.p, w.p.p, w.seg_buf.p);
+  k_spmm_rows_dot<K><<<L.grid, THREADS, 0, s>>>(e.n, e.lap_seg.row_first.p, w.seg_buf.p, e.L_diag.p, w.p.p, w.q.p,
+                                                pa);
+  k_step_alpha<K><<<1, STEP_THREADS, 0, s>>>(pa, L.grid, w.s);
   k_update_xr<K><<<L.grid, THREADS, 0, s>>>(e.n, w.p.p, w.q.p, w.x.p, w.r.p, w.s.alpha, pa);
   e.mg->apply(K, w.r.p, w.z.p, s);
   k_dot<K><<<L.grid, THREADS, 0, s>>>(e.n, w.r.p, w.z.p, pb);
-  k_step_beta<K, 1><<<1, 128, 0, s>>>(pa, L.grid, pb, L.grid, w.s);
+  k_step_beta<K><<<1, STEP_THREADS, 0, s>>>(pa, L.grid, pb, L.grid, w.s);
   k_direction<K><<<L.grid, THREADS, 0, s>>>(e.n, w.z.p, w.p.p, w.s.beta);
 }
 

@@ -263,6 +263,70 @@ __device__ __forceinline__ void warp_gather(uint32_t my_j, double my_a, uint32_t
   }
 }
 
+// The calling block sums the per-block partials [blocks][M][K] in a fixed
+// order; result into out[M*K] (shared).  Uses all threads: T/(M*K) lanes per
+// output, their sums halved pairwise down to 16 and added in order (one
+// thread adding all 1024 lanes of a one-column block took 5.6 us).
+template <int M, int K>
+__device__ __forceinline__ void redundant_finish(const double* __restrict__ partial, int blocks, double* out,
+                                                 double* scratch /* blockDim doubles */) {
+  constexpr int W = M * K;
+  int per = blockDim.x / W;  // >= 1 when blockDim >= W
+  const int o = threadIdx.x % W, g = threadIdx.x / W;
+  // the loads of U partials are issued before their sum, so a thread waits
+  // for one L2 round trip per U blocks instead of one per block
+  constexpr int U = 8;
+  double acc = 0.0;
+  if (g < per)
+    for (int b0 = g; b0 < blocks; b0 += U * per) {
+      double v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int b = b0 + u * per;
+        v[u] = b < blocks ? __ldcg(partial + size_t(b) * W + o) : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) acc += v[u];
+    }
+  scratch[threadIdx.x] = acc;
+  __syncthreads();
+  for (; per > 16; per >>= 1) {
+    if (g < per / 2) scratch[threadIdx.x] += scratch[threadIdx.x + per / 2 * W];
+    __syncthreads();
+  }
+  if (threadIdx.x < W) {
+    double s = 0.0;
+    for (int k = 0; k < per; ++k) s += scratch[k * W + threadIdx.x];
+    out[threadIdx.x] = s;
+  }
+  __syncthreads();
+}
+
+// Subtract a row's segment products (segments [s0, s1), K columns) from acc
+// in order, eight loads in flight: a hub row's hundreds of segments cost one
+// memory round trip per eight.
+template <int K, typename V>
+__device__ __forceinline__ void subtract_segments(const V* seg, uint32_t s0, uint32_t s1, int c0,
+                                                  double (&acc)[Cols<K>::CPT]) {
+  constexpr int CPT = Cols<K>::CPT, U = 8;
+  uint32_t sg = s0;
+  for (; sg + U <= s1; sg += U) {
+    double v[U][CPT];
+#pragma unroll
+    for (int u = 0; u < U; ++u) load_cols<K, V>(seg, sg + u, c0, v[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) acc[c] -= v[u][c];
+  }
+  for (; sg < s1; ++sg) {
+    double v[CPT];
+    load_cols<K, V>(seg, sg, c0, v);
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) acc[c] -= v[c];
+  }
+}
+
 // Warp-combined maximum of non-negative doubles into *slot (the bit patterns
 // of non-negative doubles order like the values).
 __device__ __forceinline__ void warp_max_into(double v, unsigned long long* slot) {
@@ -391,17 +455,17 @@ __global__ void __launch_bounds__(THREADS) k_direction(uint32_t n, const double*
   }
 }
 
-// Single-block step kernels on the per-column state.
+// Single-block step kernels of the multigrid form on the per-column state,
+// all 1024 threads on the partials (with 128 threads, one a column, the 1,184
+// partials of a column were a serial chain: 54 and 127 us an iteration at
+// K = 64 on a 10k-vertex graph; 9 and 15 us now).
+constexpr int STEP_THREADS = 1024;
+
 template <int K>
-__global__ void k_step_alpha(const double* __restrict__ partial, int blocks, PcgState s) {
-  __shared__ double pq[K];
-  // finish p.q
-  for (int j = threadIdx.x; j < K; j += blockDim.x) {
-    double acc = 0.0;
-    for (int b = 0; b < blocks; ++b) acc += partial[size_t(b) * K + j];
-    pq[j] = acc;
-  }
-  __syncthreads();
+__global__ void __launch_bounds__(STEP_THREADS) k_step_alpha(const double* __restrict__ partial, int blocks,
+                                                             PcgState s) {
+  __shared__ double pq[K], scratch[STEP_THREADS];
+  redundant_finish<1, K>(partial, blocks, pq, scratch);  // finish p.q
   for (int j = threadIdx.x; j < K; j += blockDim.x) {
     double a = 0.0;
     if (s.active[j]) {
@@ -416,25 +480,18 @@ __global__ void k_step_alpha(const double* __restrict__ partial, int blocks, Pcg
   }
 }
 
-// M = 1: partial is (r.r) only and rz is taken from a separate dot (multigrid);
-// M = 2: partial holds (r.z, r.r).
-template <int K, int M>
-__global__ void k_step_beta(const double* __restrict__ partial, int blocks, const double* __restrict__ partial_rz,
-                            int blocks_rz, PcgState s) {
+// partial: r.r of the update; partial_rz: r.z of the preconditioned residual
+template <int K>
+__global__ void __launch_bounds__(STEP_THREADS) k_step_beta(const double* __restrict__ partial, int blocks,
+                                                            const double* __restrict__ partial_rz, int blocks_rz,
+                                                            PcgState s) {
   __shared__ int cnt;
+  __shared__ double rr_s[K], rz_s[K], scratch[STEP_THREADS];
   if (threadIdx.x == 0) cnt = 0;
-  __syncthreads();
+  redundant_finish<1, K>(partial, blocks, rr_s, scratch);
+  redundant_finish<1, K>(partial_rz, blocks_rz, rz_s, scratch);
   for (int j = threadIdx.x; j < K; j += blockDim.x) {
-    double rz = 0.0, rr = 0.0;
-    if (M == 2) {
-      for (int b = 0; b < blocks; ++b) {
-        rz += partial[size_t(b) * 2 * K + j];
-        rr += partial[size_t(b) * 2 * K + K + j];
-      }
-    } else {
-      for (int b = 0; b < blocks; ++b) rr += partial[size_t(b) * K + j];
-      for (int b = 0; b < blocks_rz; ++b) rz += partial_rz[size_t(b) * K + j];
-    }
+    const double rz = rz_s[j], rr = rr_s[j];
     double be = 0.0;
     if (s.active[j]) {
       s.iters[j] += 1;

@@ -822,11 +822,11 @@ class Trainer final : public GnnTrainer {
     while (nactive > 0 && it < 1000) {
       k_spmm_dot<K><<<blocks, THREADS, 0, s>>>(n, tg.g.ptr.p, tg.g.col.p, tg.g.val.p, tg.g.diag.p, pp.p, q.p,
                                                part.p);
-      k_step_alpha<K><<<1, 128, 0, s>>>(part.p, blocks, ps);
+      k_step_alpha<K><<<1, STEP_THREADS, 0, s>>>(part.p, blocks, ps);
       k_update_xr<K><<<blocks, THREADS, 0, s>>>(n, pp.p, q.p, x.p, r.p, ps.alpha, part.p);
       mg.apply(K, r.p, z.p, s);
       k_dot<K><<<blocks, THREADS, 0, s>>>(n, r.p, z.p, part.p + size_t(blocks) * K);
-      k_step_beta<K, 1><<<1, 128, 0, s>>>(part.p, blocks, part.p + size_t(blocks) * K, blocks, ps);
+      k_step_beta<K><<<1, STEP_THREADS, 0, s>>>(part.p, blocks, part.p + size_t(blocks) * K, blocks, ps);
       k_direction<K><<<blocks, THREADS, 0, s>>>(n, z.p, pp.p, ps.beta);
       ++it;
       CK(cudaMemcpyAsync(&nactive, ps.nactive, sizeof(int), cudaMemcpyDeviceToHost, s));

@@ -61,15 +61,32 @@ __global__ void k_mg_products(uint32_t nseg, const uint32_t* __restrict__ seg_be
     double acc[CPT];
 #pragma unroll
     for (int c = 0; c < CPT; ++c) acc[c] = 0.0;
-    for (uint32_t e = seg_begin[sg]; e < seg_end[sg]; ++e) {
-      size_t u = col[e];
-      double w = val[e];
-      size_t au = PROLONG ? size_t(agg[u]) * K : 0;
+    if constexpr (TPR == 32) {
+      // one warp per segment: its columns, values and aggregates loaded
+      // lane-parallel and broadcast, so a segment waits for two index loads
+      // and its rows instead of a chain of them per entry
+      const uint32_t lane = threadIdx.x & 31, sb = seg_begin[sg], cnt = seg_end[sg] - sb;
+      uint32_t my_u = 0, my_g = 0;
+      double my_w = 0.0, my_s = 0.0;
+      if (lane < cnt) {
+        my_u = col[sb + lane];
+        my_w = val[sb + lane];
+        my_s = FIRST ? my_w * invd[my_u] : my_w;
+        if (PROLONG) my_g = agg[my_u];
+      }
+      warp_gather<K, double>(my_u, my_s, cnt, FIRST ? b : x, c0, acc);
+      if (PROLONG) warp_gather<K, double>(my_g, my_w, cnt, cx, c0, acc);
+    } else {
+      for (uint32_t e = seg_begin[sg]; e < seg_end[sg]; ++e) {
+        size_t u = col[e];
+        double w = val[e];
+        size_t au = PROLONG ? size_t(agg[u]) * K : 0;
 #pragma unroll
-      for (int c = 0; c < CPT; ++c) {
-        double y = start_value<FIRST>(x, b, invd, u, u * K + c0 + c);
-        if (PROLONG) y += cx[au + c0 + c];
-        acc[c] += w * y;
+        for (int c = 0; c < CPT; ++c) {
+          double y = start_value<FIRST>(x, b, invd, u, u * K + c0 + c);
+          if (PROLONG) y += cx[au + c0 + c];
+          acc[c] += w * y;
+        }
       }
     }
 #pragma unroll
@@ -100,9 +117,7 @@ __global__ void k_mg_finish(uint32_t n, const uint32_t* __restrict__ row_first, 
       if (PROLONG) y[c] += cx[av + c0 + c];
       ly[c] = d * y[c];
     }
-    for (uint32_t s = row_first[v]; s < row_first[v + 1]; ++s)
-#pragma unroll
-      for (int c = 0; c < CPT; ++c) ly[c] -= seg_out[size_t(s) * K + c0 + c];
+    subtract_segments<K, double>(seg_out, row_first[v], row_first[v + 1], c0, ly);
     double dv = invd[v];
 #pragma unroll
     for (int c = 0; c < CPT; ++c) {

@@ -169,37 +169,78 @@ __device__ __forceinline__ void block_reduce_cols_big(double (&v)[M][Cols<K>::CP
   __syncthreads();
 }
 
-// Every block sums the per-block partials [blocks][M][K] in the same order;
-// result into out[M*K] (shared).  Uses all threads: T/(M*K) lanes per output.
-template <int M, int K>
-__device__ __forceinline__ void redundant_finish(const double* __restrict__ partial, int blocks, double* out,
-                                                 double* scratch /* blockDim doubles */) {
-  constexpr int W = M * K;
-  const int per = blockDim.x / W;  // >= 1 when blockDim >= W
-  const int o = threadIdx.x % W, g = threadIdx.x / W;
-  // the loads of U partials are issued before their sum, so a thread waits
-  // for one L2 round trip per U blocks instead of one per block
-  constexpr int U = 8;
-  double acc = 0.0;
-  if (g < per)
-    for (int b0 = g; b0 < blocks; b0 += U * per) {
-      double v[U];
+// Products of the Laplacian's off-diagonal entries over its segments in the
+// balanced order, seg[id] = sum_e a_e x[col_e] (one warp per segment for
+// K >= 32), and the rows' finish y = diag x - sum of the row's segments with
+// the per-column dot x.y: the multigrid form's product.  One row per warp
+// walked a hub firm's thousands of entries on one warp (300 us an iteration
+// at K = 64 on a 10k-vertex firm graph of 175k entries; 40 us now).
+template <int K>
+__global__ void __launch_bounds__(THREADS) k_spmm_segments(uint32_t nseg, const uint32_t* __restrict__ ord_id,
+                                                           const uint32_t* __restrict__ ord_begin,
+                                                           const uint32_t* __restrict__ ord_end,
+                                                           const uint32_t* __restrict__ col,
+                                                           const double* __restrict__ val, const double* __restrict__ x,
+                                                           double* __restrict__ seg) {
+  constexpr int CPT = Cols<K>::CPT, TPR = Cols<K>::TPR;
+  const size_t total = size_t(nseg) * TPR, stride = size_t(gridDim.x) * blockDim.x;
+  const int c0 = int(threadIdx.x % TPR) * CPT;
+  for (size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += stride) {
+    const size_t sg = t / TPR;
+    const uint32_t b = ord_begin[sg], e = ord_end[sg];
+    double acc[CPT];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int b = b0 + u * per;
-        v[u] = b < blocks ? __ldcg(partial + size_t(b) * W + o) : 0.0;
+    for (int c = 0; c < CPT; ++c) acc[c] = 0.0;
+    if constexpr (TPR == 32) {
+      const uint32_t lane = threadIdx.x & 31;
+      uint32_t my_j = 0;
+      double my_a = 0.0;
+      if (lane < e - b) {
+        my_j = col[b + lane];
+        my_a = val[b + lane];
       }
+      warp_gather<K, double>(my_j, my_a, e - b, x, c0, acc);
+    } else {
+      for (uint32_t i = b; i < e; ++i) {
+        double xv[CPT];
+        load_cols<K, double>(x, col[i], c0, xv);
 #pragma unroll
-      for (int u = 0; u < U; ++u) acc += v[u];
+        for (int c = 0; c < CPT; ++c) acc[c] += val[i] * xv[c];
+      }
     }
-  scratch[threadIdx.x] = acc;
-  __syncthreads();
-  if (threadIdx.x < W) {
-    double s = 0.0;
-    for (int k = 0; k < per; ++k) s += scratch[k * W + threadIdx.x];
-    out[threadIdx.x] = s;
+    const size_t o = size_t(ord_id[sg]) * K + c0;
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) seg[o + c] = acc[c];
   }
-  __syncthreads();
+}
+
+template <int K>
+__global__ void __launch_bounds__(THREADS) k_spmm_rows_dot(uint32_t n, const uint32_t* __restrict__ row_first,
+                                                           const double* __restrict__ seg,
+                                                           const double* __restrict__ diag,
+                                                           const double* __restrict__ x, double* __restrict__ y,
+                                                           double* __restrict__ partial) {
+  constexpr int CPT = Cols<K>::CPT, TPR = Cols<K>::TPR;
+  double v[1][CPT];
+#pragma unroll
+  for (int c = 0; c < CPT; ++c) v[0][c] = 0.0;
+  const int c0 = int(threadIdx.x % TPR) * CPT;
+  const size_t total = size_t(n) * TPR, stride = size_t(gridDim.x) * blockDim.x;
+  for (size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += stride) {
+    const uint32_t r = uint32_t(t / TPR);
+    const double d = diag[r];
+    double xr[CPT], acc[CPT];
+    load_cols<K, double>(x, r, c0, xr);
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) acc[c] = d * xr[c];
+    subtract_segments<K, double>(seg, row_first[r], row_first[r + 1], c0, acc);
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) {
+      y[size_t(r) * K + c0 + c] = acc[c];
+      v[0][c] += acc[c] * xr[c];
+    }
+  }
+  block_reduce_cols<K, 1>(v, partial);
 }
 
 // V is the storage type of the Laplacian values and of the iteration vectors
