@@ -101,8 +101,8 @@ namespace {
 
 constexpr int GNN_THREADS = 256;
 constexpr int GNN_GRAD_BLOCKS = 148;
-constexpr int WGRAD_PER_THREAD = 17;  // (64 + 1) x 64 outputs over 256 threads
-constexpr int ENERGY_BLOCKS = 64;
+constexpr int WGRAD_ROWS = 16;        // rows of a weight-gradient tile
+constexpr int ENERGY_BLOCKS = 592;    // at most, one vertex at a time each (4 per SM)
 
 int gnn_blocks(size_t work) {
   size_t b = (work + GNN_THREADS - 1) / GNN_THREADS;
@@ -148,21 +148,61 @@ __global__ void k_gnn_aggregate(uint32_t n, const uint32_t* __restrict__ ptr, co
 }
 
 
-// dH[u][i] += sum_v (w_uv / d_v) T[v][i]   (transpose of the aggregation)
-__global__ void k_gnn_aggregate_t(uint32_t n, int in, const uint32_t* __restrict__ ptr,
-                                  const uint32_t* __restrict__ col, const double* __restrict__ val,
-                                  const double* __restrict__ diag, const float* __restrict__ T,
-                                  float* __restrict__ dH) {
-  size_t total = size_t(n) * in;
-  for (size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += size_t(gridDim.x) * blockDim.x) {
-    size_t u = t / in;
-    int i = int(t % in);
-    float acc = 0.0f;
-    for (uint32_t e = ptr[u]; e < ptr[u + 1]; ++e) {
-      uint32_t v = col[e];
-      acc += float(val[e] / diag[v]) * T[size_t(v) * in + i];
+// One block per vertex: sum over the vertex's edges of term(e, col_e, t) for
+// the columns t < P, returned by thread t.  The eight warps take four edges
+// each per sweep (their rows are loaded together), a lane holds the columns
+// lane, lane + 32, ..; the warps' sums are added in order, in FP64.  A firm
+// graph's hubs hold thousands of edges, so one thread or warp per vertex waits
+// on the longest row (1,500 firms, 48 pairs, the whole pass over the network
+// and the pairs: 4.2 ms with a thread a vertex, 0.5 ms so).
+constexpr int ROW_WARPS = GNN_THREADS / 32;
+
+template <int PER, typename Term>
+__device__ __forceinline__ double block_row_sum(uint32_t begin, uint32_t end, const uint32_t* __restrict__ col,
+                                                Term term, int P, double (*sm)[PER * 32]) {
+  constexpr int U = 4;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double acc[PER];
+#pragma unroll
+  for (int k = 0; k < PER; ++k) acc[k] = 0.0;
+  for (uint32_t e0 = begin + uint32_t(warp) * U; e0 < end; e0 += ROW_WARPS * U) {
+    double x[U][PER];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool on = e0 + u < end;
+      const uint32_t c = on ? col[e0 + u] : 0;
+#pragma unroll
+      for (int k = 0; k < PER; ++k) x[u][k] = on && lane + 32 * k < P ? term(e0 + u, c, lane + 32 * k) : 0.0;
     }
-    dH[t] += acc;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int k = 0; k < PER; ++k) acc[k] += x[u][k];
+  }
+  __syncthreads();  // the previous vertex's sums have been read
+#pragma unroll
+  for (int k = 0; k < PER; ++k) sm[warp][lane + 32 * k] = acc[k];
+  __syncthreads();
+  double sum = 0.0;
+  if (int(threadIdx.x) < P)
+#pragma unroll
+    for (int w = 0; w < ROW_WARPS; ++w) sum += sm[w][threadIdx.x];
+  return sum;
+}
+
+// dH[u][i] += sum_v (w_uv / d_v) T[v][i]   (transpose of the aggregation)
+__global__ void __launch_bounds__(GNN_THREADS) k_gnn_aggregate_t(uint32_t n, const uint32_t* __restrict__ ptr,
+                                                                 const uint32_t* __restrict__ col,
+                                                                 const double* __restrict__ val,
+                                                                 const double* __restrict__ diag,
+                                                                 const float* __restrict__ T, float* __restrict__ dH) {
+  __shared__ double sm[ROW_WARPS][GNN_WIDTH];
+  for (uint32_t u = blockIdx.x; u < n; u += gridDim.x) {
+    const double sum = block_row_sum<GNN_WIDTH / 32>(
+        ptr[u], ptr[u + 1], col,
+        [&](uint32_t e, uint32_t c, int i) { return val[e] / diag[c] * double(T[size_t(c) * GNN_WIDTH + i]); },
+        GNN_WIDTH, sm);
+    if (threadIdx.x < GNN_WIDTH) dH[size_t(u) * GNN_WIDTH + threadIdx.x] += float(sum);
   }
 }
 
@@ -235,63 +275,93 @@ __global__ void k_gnn_relu_back(size_t total, const float* __restrict__ dH, cons
     dZ[t] = Hout[t] > 0.0f ? dH[t] : 0.0f;
 }
 
-// dX[v][i] = sum_j dZ[v][j] W[i][j]   (W is in x 64, BF16); accumulate when add
-__global__ void k_gnn_input_grad(uint32_t n, int in, const float* __restrict__ dZ,
-                                 const __nv_bfloat16* __restrict__ W, float* __restrict__ dX, int add) {
-  __shared__ __nv_bfloat16 sw[GNN_WIDTH * GNN_WIDTH];
-  for (int t = threadIdx.x; t < in * GNN_WIDTH; t += blockDim.x) sw[t] = W[t];
+// dX[v][i] = sum_j dZ[v][j] Ws[i][j] and T[v][i] = sum_j dZ[v][j] Wn[i][j]
+// (64 x 64, BF16).  The weights sit in shared memory column by column, so the
+// threads of a vertex read consecutive entries (row by row, 32 threads met in
+// one bank).
+__global__ void __launch_bounds__(GNN_THREADS) k_gnn_input_grad(uint32_t n, const float* __restrict__ dZ,
+                                                                const __nv_bfloat16* __restrict__ Ws,
+                                                                const __nv_bfloat16* __restrict__ Wn,
+                                                                float* __restrict__ dX, float* __restrict__ T) {
+  __shared__ float sw[2][GNN_WIDTH][GNN_WIDTH + 1];
+  for (int t = threadIdx.x; t < GNN_WIDTH * GNN_WIDTH; t += blockDim.x) {
+    sw[0][t % GNN_WIDTH][t / GNN_WIDTH] = __bfloat162float(Ws[t]);
+    sw[1][t % GNN_WIDTH][t / GNN_WIDTH] = __bfloat162float(Wn[t]);
+  }
   __syncthreads();
-  size_t total = size_t(n) * in;
+  const size_t total = size_t(n) * GNN_WIDTH;
   for (size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += size_t(gridDim.x) * blockDim.x) {
-    size_t v = t / in;
-    int i = int(t % in);
-    float acc = 0.0f;
-    for (int j = 0; j < GNN_WIDTH; ++j) acc += dZ[v * GNN_WIDTH + j] * __bfloat162float(sw[i * GNN_WIDTH + j]);
-    dX[t] = add ? dX[t] + acc : acc;
-  }
-}
-
-// Weight gradients: partial[blk][i][j] = sum over the block's rows of
-// A[v][i] B[v][j] (A is n x in, B is n x out); with bias, partial row `in`
-// holds sum of B[v][j].  Rows split into contiguous ranges per block.
-__global__ void k_gnn_wgrad(uint32_t n, int in, int out, const float* __restrict__ A, const float* __restrict__ B,
-                            int bias, float* __restrict__ partial) {
-  const int width = (in + bias) * out;
-  extern __shared__ float sh[];
-  float* sa = sh;                  // [in]
-  float* sb = sh + GNN_WIDTH;      // [out]
-  uint32_t per = (n + gridDim.x - 1) / gridDim.x;
-  uint32_t r0 = blockIdx.x * per, r1 = min(n, r0 + per);
-  float acc[WGRAD_PER_THREAD];
-#pragma unroll
-  for (int q = 0; q < WGRAD_PER_THREAD; ++q) acc[q] = 0.0f;
-  for (uint32_t v = r0; v < r1; ++v) {
-    __syncthreads();
-    for (int t = threadIdx.x; t < in; t += blockDim.x) sa[t] = A[size_t(v) * in + t];
-    for (int t = threadIdx.x; t < out; t += blockDim.x) sb[t] = B[size_t(v) * out + t];
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < WGRAD_PER_THREAD; ++q) {
-      int o = threadIdx.x + q * blockDim.x;
-      if (o < width) {
-        int i = o / out, j = o % out;
-        acc[q] += (i < in ? sa[i] : 1.0f) * sb[j];
-      }
+    const int i = int(t % GNN_WIDTH);
+    const float4* z = reinterpret_cast<const float4*>(dZ + t / GNN_WIDTH * GNN_WIDTH);
+    float a = 0.0f, b = 0.0f;
+#pragma unroll 4
+    for (int j = 0; j < GNN_WIDTH / 4; ++j) {
+      const float4 v = z[j];
+      a += v.x * sw[0][4 * j][i] + v.y * sw[0][4 * j + 1][i] + v.z * sw[0][4 * j + 2][i] + v.w * sw[0][4 * j + 3][i];
+      b += v.x * sw[1][4 * j][i] + v.y * sw[1][4 * j + 1][i] + v.z * sw[1][4 * j + 2][i] + v.w * sw[1][4 * j + 3][i];
     }
-  }
-#pragma unroll
-  for (int q = 0; q < WGRAD_PER_THREAD; ++q) {
-    int o = threadIdx.x + q * blockDim.x;
-    if (o < width) partial[size_t(blockIdx.x) * width + o] = acc[q];
+    dX[t] = a;
+    T[t] = b;
   }
 }
 
-// grad[o] = sum over blocks (in order) of partial[blk][o]
-__global__ void k_gnn_wgrad_finish(int blocks, int width, const float* __restrict__ partial,
-                                   float* __restrict__ grad) {
-  for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < width; o += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int b = 0; b < blocks; ++b) s += partial[size_t(b) * width + o];
+// Weight gradients of a layer, its SETS inputs (the vertices' own and the
+// aggregated ones) and its bias at once: partial[blk][i][j] = sum over the
+// block's rows of A_i B_j with i over A[0] (IN), A[1] (IN, when SETS = 2) and
+// the bias (1), the layout of the parameters.  Rows split into contiguous
+// ranges per block, WGRAD_ROWS of them staged at a time (one barrier pair per
+// tile instead of per row).
+template <int IN, int OUT, int SETS>
+__global__ void __launch_bounds__(GNN_THREADS) k_gnn_wgrad(uint32_t n, const float* __restrict__ A0,
+                                                           const float* __restrict__ A1, const float* __restrict__ B,
+                                                           float* __restrict__ partial) {
+  constexpr int ROWS = SETS * IN + 1, WIDTH = ROWS * OUT, PER = (WIDTH + GNN_THREADS - 1) / GNN_THREADS;
+  __shared__ float sa[WGRAD_ROWS][ROWS], sb[WGRAD_ROWS][OUT];
+  const uint32_t per = (n + gridDim.x - 1) / gridDim.x;
+  const uint32_t r0 = min(n, blockIdx.x * per), r1 = min(n, r0 + per);
+  float acc[PER];
+#pragma unroll
+  for (int q = 0; q < PER; ++q) acc[q] = 0.0f;
+  for (uint32_t v0 = r0; v0 < r1; v0 += WGRAD_ROWS) {
+    const int rows = int(min(r1 - v0, uint32_t(WGRAD_ROWS)));
+    __syncthreads();
+    for (int t = threadIdx.x; t < rows * ROWS; t += blockDim.x) {
+      const int r = t / ROWS, i = t % ROWS;
+      sa[r][i] = i < IN ? A0[size_t(v0 + r) * IN + i] : i < SETS * IN ? A1[size_t(v0 + r) * IN + i - IN] : 1.0f;
+    }
+    for (int t = threadIdx.x; t < rows * OUT; t += blockDim.x) sb[t / OUT][t % OUT] = B[size_t(v0) * OUT + t];
+    __syncthreads();
+    for (int r = 0; r < rows; ++r)
+#pragma unroll
+      for (int q = 0; q < PER; ++q) {
+        const int o = int(threadIdx.x) + q * GNN_THREADS;
+        if (o < WIDTH) acc[q] += sa[r][o / OUT] * sb[r][o % OUT];
+      }
+  }
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    const int o = int(threadIdx.x) + q * GNN_THREADS;
+    if (o < WIDTH) partial[size_t(blockIdx.x) * WIDTH + o] = acc[q];
+  }
+}
+
+// grad[o] = sum over blocks of partial[blk][o]: eight lanes an output, their
+// sums added in order.
+constexpr int WFINISH_OUT = 32;
+__global__ void __launch_bounds__(GNN_THREADS) k_gnn_wgrad_finish(int blocks, int width,
+                                                                  const float* __restrict__ partial,
+                                                                  float* __restrict__ grad) {
+  constexpr int LANES = GNN_THREADS / WFINISH_OUT;
+  __shared__ double sm[LANES][WFINISH_OUT];
+  const int o = blockIdx.x * WFINISH_OUT + threadIdx.x % WFINISH_OUT, g = threadIdx.x / WFINISH_OUT;
+  double s = 0.0;
+  if (o < width)
+#pragma unroll 4
+    for (int b = g; b < blocks; b += LANES) s += partial[size_t(b) * width + o];
+  sm[g][threadIdx.x % WFINISH_OUT] = s;
+  __syncthreads();
+  if (g == 0 && o < width) {
+    for (int k = 1; k < LANES; ++k) s += sm[k][threadIdx.x];
     grad[o] = float(s);
   }
 }
@@ -325,25 +395,27 @@ __global__ void k_adam(size_t n, float* __restrict__ p, const float* __restrict_
 
 // Forward of the degree-1 stage on the pairs (P columns, vertex-interleaved),
 // with y_0 = r / d:  U = s y_0 (= (s/d) r),  AU = A U,  Z = a y_0 + (s/d) AU.
-__global__ void k_pair_sym_u(uint32_t n, int P, const float* __restrict__ C, const float* __restrict__ Y0,
-                             float* __restrict__ U) {
-  size_t total = size_t(n) * P;
-  for (size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += size_t(gridDim.x) * blockDim.x)
-    U[t] = C[(t / P) * GNN_OUT + 1] * Y0[t];
-}
-
-__global__ void k_pair_sym_z(uint32_t n, int P, const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
-                             const double* __restrict__ val, const double* __restrict__ diag,
-                             const float* __restrict__ C, const float* __restrict__ Y0, const float* __restrict__ U,
-                             float* __restrict__ AU, float* __restrict__ Z) {
-  size_t total = size_t(n) * P;
-  for (size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += size_t(gridDim.x) * blockDim.x) {
-    size_t v = t / P;
-    int j = int(t % P);
-    double acc = 0.0;
-    for (uint32_t e = ptr[v]; e < ptr[v + 1]; ++e) acc += val[e] * double(U[size_t(col[e]) * P + j]);
-    AU[t] = float(acc);
-    Z[t] = float(double(C[v * GNN_OUT]) * double(Y0[t]) + double(C[v * GNN_OUT + 1]) / diag[v] * acc);
+template <int PER>
+__global__ void __launch_bounds__(GNN_THREADS) k_pair_sym_z(uint32_t n, int P, const uint32_t* __restrict__ ptr,
+                                                            const uint32_t* __restrict__ col,
+                                                            const double* __restrict__ val,
+                                                            const double* __restrict__ diag,
+                                                            const float* __restrict__ C, const float* __restrict__ Y0,
+                                                            float* __restrict__ AU, float* __restrict__ Z) {
+  __shared__ double sm[ROW_WARPS][PER * 32];
+  for (uint32_t v = blockIdx.x; v < n; v += gridDim.x) {
+    const double acc = block_row_sum<PER>(
+        ptr[v], ptr[v + 1], col,
+        [&](uint32_t e, uint32_t c, int j) {
+          return val[e] * double(C[size_t(c) * GNN_OUT + 1] * Y0[size_t(c) * P + j]);
+        },
+        P, sm);
+    if (int(threadIdx.x) < P) {
+      const size_t t = size_t(v) * P + threadIdx.x;
+      AU[t] = float(acc);
+      Z[t] = float(double(C[size_t(v) * GNN_OUT]) * double(Y0[t]) +
+                   double(C[size_t(v) * GNN_OUT + 1]) / diag[v] * acc);
+    }
   }
 }
 
@@ -364,64 +436,125 @@ __global__ void k_pair_sym_g(uint32_t n, int P, const float* __restrict__ C, con
   }
 }
 
-__global__ void k_pair_sym_grad(uint32_t n, int P, const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
-                                const double* __restrict__ val, const double* __restrict__ diag,
-                                const float* __restrict__ Craw, const float* __restrict__ C,
-                                const float* __restrict__ Y0, const float* __restrict__ AU,
-                                const float* __restrict__ G, const float* __restrict__ Wv,
-                                float* __restrict__ dCraw) {
-  for (size_t v = size_t(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += size_t(gridDim.x) * blockDim.x) {
+template <int PER>
+__global__ void __launch_bounds__(GNN_THREADS) k_pair_sym_grad(
+    uint32_t n, int P, const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
+    const double* __restrict__ val, const double* __restrict__ diag, const float* __restrict__ Craw,
+    const float* __restrict__ C, const float* __restrict__ Y0, const float* __restrict__ AU,
+    const float* __restrict__ G, const float* __restrict__ Wv, float* __restrict__ dCraw) {
+  __shared__ double sm[ROW_WARPS][PER * 32];
+  __shared__ double part[ROW_WARPS][2];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (uint32_t v = blockIdx.x; v < n; v += gridDim.x) {
+    const double aw = block_row_sum<PER>(
+        ptr[v], ptr[v + 1], col,
+        [&](uint32_t e, uint32_t c, int j) { return val[e] * double(Wv[size_t(c) * P + j]); }, P, sm);
     double da = 0.0, ds = 0.0;
     const double dv = diag[v];
-    for (int j = 0; j < P; ++j) {
-      size_t t = v * P + j;
-      double aw = 0.0;
-      for (uint32_t e = ptr[v]; e < ptr[v + 1]; ++e) aw += val[e] * double(Wv[size_t(col[e]) * P + j]);
-      da += double(G[t]) * double(Y0[t]);
-      ds += double(G[t]) * double(AU[t]) / dv + double(Y0[t]) * aw;
+    if (int(threadIdx.x) < P) {
+      const size_t t = size_t(v) * P + threadIdx.x;
+      da = double(G[t]) * double(Y0[t]);
+      ds = double(G[t]) * double(AU[t]) / dv + double(Y0[t]) * aw;
     }
-    const double sv = double(C[v * GNN_OUT + 1]);
-    ds += 2.0 * sv * da;
-    dCraw[v * GNN_OUT + 0] = float(da * double(sigmoidf(Craw[v * GNN_OUT + 0])));
-    dCraw[v * GNN_OUT + 1] = float(ds * double(sigmoidf(Craw[v * GNN_OUT + 1])));
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      da += __shfl_xor_sync(0xffffffffu, da, off);
+      ds += __shfl_xor_sync(0xffffffffu, ds, off);
+    }
+    if (lane == 0) {
+      part[warp][0] = da;
+      part[warp][1] = ds;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < ROW_WARPS; ++w) {
+        da += part[w][0];
+        ds += part[w][1];
+      }
+      ds += 2.0 * double(C[size_t(v) * GNN_OUT + 1]) * da;
+      dCraw[size_t(v) * GNN_OUT + 0] = float(da * double(sigmoidf(Craw[size_t(v) * GNN_OUT + 0])));
+      dCraw[size_t(v) * GNN_OUT + 1] = float(ds * double(sigmoidf(Craw[size_t(v) * GNN_OUT + 1])));
+    }
+    // part is written again only after block_row_sum's barriers
   }
 }
 
 // LZ = L Z; R = d Y_0 (the residual); partial[blk][0][j] = sum_v Z R,
-// partial[blk][1][j] = sum_v Z LZ.  Block sums in a fixed order.
-__global__ void k_pair_energy(uint32_t n, int P, const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
-                              const double* __restrict__ val, const double* __restrict__ diag,
-                              const float* __restrict__ Z, const float* __restrict__ Y0, float* __restrict__ LZ,
-                              float* __restrict__ R, double* __restrict__ partial) {
-  extern __shared__ double shd[];  // [blockDim][2]
-  size_t total = size_t(n) * P;
-  for (int j = 0; j < P; ++j) {
-    double a = 0.0, b = 0.0;
-    for (size_t v = size_t(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += size_t(gridDim.x) * blockDim.x) {
-      size_t t = v * P + j;
-      float acc = float(diag[v]) * Z[t];
-      for (uint32_t e = ptr[v]; e < ptr[v + 1]; ++e) acc -= float(val[e]) * Z[size_t(col[e]) * P + j];
-      float r = float(diag[v]) * Y0[t];
+// partial[blk][1][j] = sum_v Z LZ over the block's vertices, one vertex at a
+// time.  The rows of Z are staged in shared memory ENERGY_TILE values at a
+// time by all threads; thread j then subtracts column j's products in edge
+// order (a smooth pair's L Z is a small difference, so its rounding shows in
+// the gradient: the order is part of the result).
+constexpr int ENERGY_TILE = 3072;
+__global__ void __launch_bounds__(GNN_THREADS) k_pair_energy(uint32_t n, int P, const uint32_t* __restrict__ ptr,
+                                                             const uint32_t* __restrict__ col,
+                                                             const double* __restrict__ val,
+                                                             const double* __restrict__ diag,
+                                                             const float* __restrict__ Z,
+                                                             const float* __restrict__ Y0, float* __restrict__ LZ,
+                                                             float* __restrict__ R, double* __restrict__ partial) {
+  __shared__ float tile[ENERGY_TILE], weight[ENERGY_TILE / 8];
+  const int edges = min(ENERGY_TILE / P, ENERGY_TILE / 8), j = int(threadIdx.x);
+  double a = 0.0, b = 0.0;
+  for (uint32_t v = blockIdx.x; v < n; v += gridDim.x) {
+    const uint32_t end = ptr[v + 1];
+    const float d = float(diag[v]), z = j < P ? Z[size_t(v) * P + j] : 0.0f;
+    float acc = d * z;
+    for (uint32_t e0 = ptr[v]; e0 < end; e0 += uint32_t(edges)) {
+      const int cnt = int(min(end - e0, uint32_t(edges)));
+      __syncthreads();
+      for (int t = j; t < cnt * P; t += GNN_THREADS) tile[t] = Z[size_t(col[e0 + t / P]) * P + t % P];
+      for (int t = j; t < cnt; t += GNN_THREADS) weight[t] = float(val[e0 + t]);
+      __syncthreads();
+      if (j < P)
+#pragma unroll 8
+        for (int i = 0; i < cnt; ++i) acc -= weight[i] * tile[i * P + j];
+    }
+    if (j < P) {
+      const size_t t = size_t(v) * P + j;
+      const float r = d * Y0[t];
       LZ[t] = acc;
       R[t] = r;
-      a += double(Z[t]) * double(r);
-      b += double(Z[t]) * double(acc);
+      a += double(z) * double(r);
+      b += double(z) * double(acc);
     }
-    shd[threadIdx.x * 2] = a;
-    shd[threadIdx.x * 2 + 1] = b;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double sa = 0.0, sb = 0.0;
-      for (int q = 0; q < int(blockDim.x); ++q) {
-        sa += shd[q * 2];
-        sb += shd[q * 2 + 1];
-      }
-      partial[(size_t(blockIdx.x) * 2) * P + j] = sa;
-      partial[(size_t(blockIdx.x) * 2 + 1) * P + j] = sb;
+  }
+  if (j < P) {
+    partial[size_t(blockIdx.x) * 2 * P + j] = a;
+    partial[(size_t(blockIdx.x) * 2 + 1) * P + j] = b;
+  }
+}
+
+// One block per pair: its two energies over the blocks of k_pair_energy, its
+// loss term and the coefficients (s1, s2) of dloss/dZ = s1 R + s2 LZ.
+__global__ void __launch_bounds__(GNN_THREADS) k_pair_scale(int blocks, int P, const double* __restrict__ partial,
+                                                            const float* __restrict__ ele, float* __restrict__ s12,
+                                                            double* __restrict__ terms) {
+  __shared__ double sa[GNN_THREADS], sb[GNN_THREADS];
+  const int j = blockIdx.x;
+  double a = 0.0, b = 0.0;
+  for (int k = threadIdx.x; k < blocks; k += GNN_THREADS) {
+    a += partial[size_t(k) * 2 * P + j];
+    b += partial[(size_t(k) * 2 + 1) * P + j];
+  }
+  sa[threadIdx.x] = a;
+  sb[threadIdx.x] = b;
+  __syncthreads();
+  for (int w = GNN_THREADS / 2; w > 0; w >>= 1) {
+    if (int(threadIdx.x) < w) {
+      sa[threadIdx.x] += sa[threadIdx.x + w];
+      sb[threadIdx.x] += sb[threadIdx.x + w];
     }
     __syncthreads();
   }
-  (void)total;
+  if (threadIdx.x != 0) return;
+  a = sa[0];
+  b = sb[0];
+  const double e = double(ele[j]);
+  const bool on = e > 0.0 && b > 0.0;
+  terms[j] = on ? 1.0 - a * a / (e * b) : 0.0;
+  s12[j] = on ? float(-2.0 * a / (double(P) * e * b)) : 0.0f;
+  s12[P + j] = on ? float(2.0 * a * a / (double(P) * e * b * b)) : 0.0f;
 }
 
 // y_0 = r / d  (P columns, double in, float out)
@@ -675,11 +808,11 @@ __global__ void k_trainer_init(const double* __restrict__ partial_rz, const doub
 struct TrainGraph {
   GraphData g;
   int P = 0;                 // pairs
-  DBuf<float> Y, E, Z, LZ, R, s12, U, AU, G, Wv, dCraw;
+  DBuf<float> Y, E, Z, LZ, R, s12, AU, G, Wv, dCraw, ele;
   std::vector<float> ELE;    // host copy of the energy norms
   DBuf<float> dH[2], dZ, T;  // backward temporaries (n x 64)
   DBuf<float> partial;       // weight-gradient partials
-  DBuf<double> epart;
+  DBuf<double> epart, terms;  // per-block energies, loss terms of the pairs
 };
 
 class Trainer final : public GnnTrainer {
@@ -919,93 +1052,89 @@ class Trainer final : public GnnTrainer {
     tg->Y.alloc(plane);
     k_pair_basis0<<<gnn_blocks(plane), GNN_THREADS, 0, s>>>(n, P, Rd.p, tg->g.diag.p, tg->Y.p);
     upload(tg->E, E, s, h2d);
-    for (auto* b : {&tg->Z, &tg->LZ, &tg->R, &tg->U, &tg->AU, &tg->G, &tg->Wv}) b->alloc(plane);
+    for (auto* b : {&tg->Z, &tg->LZ, &tg->R, &tg->AU, &tg->G, &tg->Wv}) b->alloc(plane);
     tg->s12.alloc(size_t(2) * P);
     tg->dCraw.alloc(size_t(n) * GNN_OUT);
     for (auto& d : tg->dH) d.alloc(size_t(n) * GNN_WIDTH);
     tg->dZ.alloc(size_t(n) * GNN_WIDTH);
     tg->T.alloc(size_t(n) * GNN_WIDTH);
-    tg->partial.alloc(size_t(GNN_GRAD_BLOCKS) * (GNN_WIDTH + 1) * GNN_WIDTH);
+    tg->partial.alloc(size_t(GNN_GRAD_BLOCKS) * (2 * GNN_WIDTH + 1) * GNN_WIDTH);
+    tg->terms.alloc(P);
+    upload(tg->ele, tg->ELE, s, h2d);
     tg->epart.alloc(size_t(ENERGY_BLOCKS) * 2 * P);
     CK(cudaStreamSynchronize(s));
     graphs_.push_back(std::move(tg));
   }
 
-  // weight gradient of A' B (+ bias row) into grad[off ...]
-  void wgrad(uint32_t n, int in, int out, const float* A, const float* B, int bias, TrainGraph& tg, size_t off) {
-    int width = (in + bias) * out;
-    if (width > WGRAD_PER_THREAD * GNN_THREADS)
-      fail(INTERNAL_INVARIANT_FAILED, "learned_train", "weight block too wide");
-    k_gnn_wgrad<<<GNN_GRAD_BLOCKS, GNN_THREADS, 2 * GNN_WIDTH * sizeof(float), s>>>(n, in, out, A, B, bias,
-                                                                                   tg.partial.p);
-    k_gnn_wgrad_finish<<<(width + 255) / 256, 256, 0, s>>>(GNN_GRAD_BLOCKS, width, tg.partial.p, grad.p + off);
+  // weight gradients of a layer (its inputs A0 and, with SETS = 2, A1, and the
+  // bias) into grad[off ...]
+  template <int IN, int OUT, int SETS>
+  void wgrad(uint32_t n, const float* A0, const float* A1, const float* B, TrainGraph& tg, size_t off) {
+    constexpr int width = (SETS * IN + 1) * OUT;
+    k_gnn_wgrad<IN, OUT, SETS><<<GNN_GRAD_BLOCKS, GNN_THREADS, 0, s>>>(n, A0, A1, B, tg.partial.p);
+    k_gnn_wgrad_finish<<<(width + WFINISH_OUT - 1) / WFINISH_OUT, GNN_THREADS, 0, s>>>(GNN_GRAD_BLOCKS, width,
+                                                                                      tg.partial.p, grad.p + off);
+  }
+
+  // the pair passes: Z, the energies and loss terms, and the head's gradient
+  template <int PER>
+  void pair_passes(TrainGraph& tg) {
+    GraphData& g = tg.g;
+    const uint32_t n = g.n;
+    const int P = tg.P, rows = int(std::min<uint32_t>(n, 148 * 8)), eblocks = int(std::min<uint32_t>(n, ENERGY_BLOCKS));
+    k_pair_sym_z<PER><<<rows, GNN_THREADS, 0, s>>>(n, P, g.ptr.p, g.col.p, g.val.p, g.diag.p, g.C.p, tg.Y.p, tg.AU.p,
+                                                   tg.Z.p);
+    k_pair_energy<<<eblocks, GNN_THREADS, 0, s>>>(n, P, g.ptr.p, g.col.p, g.val.p, g.diag.p, tg.Z.p, tg.Y.p,
+                                                  tg.LZ.p, tg.R.p, tg.epart.p);
+    k_pair_scale<<<P, GNN_THREADS, 0, s>>>(eblocks, P, tg.epart.p, tg.ele.p, tg.s12.p, tg.terms.p);
+    k_pair_sym_g<<<gnn_blocks(size_t(n) * P), GNN_THREADS, 0, s>>>(n, P, g.C.p, g.diag.p, tg.R.p, tg.LZ.p, tg.s12.p,
+                                                                   tg.G.p, tg.Wv.p);
+    k_pair_sym_grad<PER><<<rows, GNN_THREADS, 0, s>>>(n, P, g.ptr.p, g.col.p, g.val.p, g.diag.p, g.Craw.p, g.C.p,
+                                                      tg.Y.p, tg.AU.p, tg.G.p, tg.Wv.p, tg.dCraw.p);
   }
 
   double loss_and_grad(TrainGraph& tg) {
     GraphData& g = tg.g;
     const uint32_t n = g.n;
     const int P = tg.P;
-    size_t plane = size_t(n) * P;
     refresh_bf16(p, s);
     forward(g, p, s);
-    k_pair_sym_u<<<gnn_blocks(plane), GNN_THREADS, 0, s>>>(n, P, g.C.p, tg.Y.p, tg.U.p);
-    k_pair_sym_z<<<gnn_blocks(plane), GNN_THREADS, 0, s>>>(n, P, g.ptr.p, g.col.p, g.val.p, g.diag.p, g.C.p, tg.Y.p,
-                                                           tg.U.p, tg.AU.p, tg.Z.p);
-    k_pair_energy<<<ENERGY_BLOCKS, GNN_THREADS, 2 * GNN_THREADS * sizeof(double), s>>>(
-        n, P, g.ptr.p, g.col.p, g.val.p, g.diag.p, tg.Z.p, tg.Y.p, tg.LZ.p, tg.R.p, tg.epart.p);
-    std::vector<double> ep(size_t(ENERGY_BLOCKS) * 2 * P);
-    CK(cudaMemcpyAsync(ep.data(), tg.epart.p, ep.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    double loss = 0.0;
-    std::vector<float> s12(size_t(2) * P, 0.0f);
-    for (int j = 0; j < P; ++j) {
-      double a = 0.0, b = 0.0;
-      for (int bl = 0; bl < ENERGY_BLOCKS; ++bl) {
-        a += ep[(size_t(bl) * 2) * P + j];
-        b += ep[(size_t(bl) * 2 + 1) * P + j];
-      }
-      double ele = tg.ELE[j];
-      if (ele > 0.0 && b > 0.0) {
-        loss += 1.0 - a * a / (ele * b);
-        s12[j] = float(-2.0 * a / (double(P) * ele * b));
-        s12[P + j] = float(2.0 * a * a / (double(P) * ele * b * b));
-      }
+    switch ((P + 31) / 32) {  // P = 24, 48, 96 or 192
+      case 1: pair_passes<1>(tg); break;
+      case 2: pair_passes<2>(tg); break;
+      case 3: pair_passes<3>(tg); break;
+      default: pair_passes<6>(tg); break;
     }
-    loss /= P;
-    CK(cudaMemcpyAsync(tg.s12.p, s12.data(), s12.size() * sizeof(float), cudaMemcpyHostToDevice, s));
-    k_pair_sym_g<<<gnn_blocks(plane), GNN_THREADS, 0, s>>>(n, P, g.C.p, g.diag.p, tg.R.p, tg.LZ.p, tg.s12.p, tg.G.p,
-                                                           tg.Wv.p);
-    k_pair_sym_grad<<<gnn_blocks(n), GNN_THREADS, 0, s>>>(n, P, g.ptr.p, g.col.p, g.val.p, g.diag.p, g.Craw.p, g.C.p,
-                                                          tg.Y.p, tg.AU.p, tg.G.p, tg.Wv.p, tg.dCraw.p);
     // head
     size_t oh = gnn_layer_offset(GNN_LAYERS);
     k_gnn_head_back<<<gnn_blocks(size_t(n) * GNN_WIDTH), GNN_THREADS, 0, s>>>(n, tg.dCraw.p, p.bf.p + oh,
                                                                               tg.dH[0].p);
-    wgrad(n, GNN_WIDTH, GNN_OUT, g.H[GNN_LAYERS - 1].p, tg.dCraw.p, 1, tg, oh);
+    wgrad<GNN_WIDTH, GNN_OUT, 1>(n, g.H[GNN_LAYERS - 1].p, nullptr, tg.dCraw.p, tg, oh);
     // layers, last to first; dH[cur] holds the gradient of the layer's output
     int cur = 0;
     for (int l = GNN_LAYERS - 1; l >= 0; --l) {
-      int w = layer_in(l);
       size_t o = gnn_layer_offset(l);
-      const float* in = l == 0 ? g.X.p : g.H[l - 1].p;
       k_gnn_relu_back<<<gnn_blocks(size_t(n) * GNN_WIDTH), GNN_THREADS, 0, s>>>(size_t(n) * GNN_WIDTH, tg.dH[cur].p,
                                                                                g.H[l].p, tg.dZ.p);
-      // Ws (with the bias as its extra row)
-      wgrad(n, w, GNN_WIDTH, in, tg.dZ.p, 0, tg, o);
-      wgrad(n, w, GNN_WIDTH, g.S[l].p, tg.dZ.p, 1, tg, o + size_t(w) * GNN_WIDTH);
-      if (l > 0) {
-        int nxt = 1 - cur;
-        k_gnn_input_grad<<<gnn_blocks(size_t(n) * w), GNN_THREADS, 0, s>>>(n, w, tg.dZ.p, p.bf.p + o, tg.dH[nxt].p,
-                                                                          0);
-        k_gnn_input_grad<<<gnn_blocks(size_t(n) * w), GNN_THREADS, 0, s>>>(
-            n, w, tg.dZ.p, p.bf.p + o + size_t(w) * GNN_WIDTH, tg.T.p, 0);
-        k_gnn_aggregate_t<<<gnn_blocks(size_t(n) * w), GNN_THREADS, 0, s>>>(n, w, g.ptr.p, g.col.p, g.val.p,
-                                                                           g.diag.p, tg.T.p, tg.dH[nxt].p);
-        cur = nxt;
+      if (l == 0) {
+        wgrad<GNN_FEATURES, GNN_WIDTH, 2>(n, g.X.p, g.S[0].p, tg.dZ.p, tg, o);
+        break;
       }
+      wgrad<GNN_WIDTH, GNN_WIDTH, 2>(n, g.H[l - 1].p, g.S[l].p, tg.dZ.p, tg, o);
+      const int nxt = 1 - cur;
+      k_gnn_input_grad<<<gnn_blocks(size_t(n) * GNN_WIDTH), GNN_THREADS, 0, s>>>(
+          n, tg.dZ.p, p.bf.p + o, p.bf.p + o + size_t(GNN_WIDTH) * GNN_WIDTH, tg.dH[nxt].p, tg.T.p);
+      k_gnn_aggregate_t<<<int(std::min<uint32_t>(n, 148 * 8)), GNN_THREADS, 0, s>>>(n, g.ptr.p, g.col.p, g.val.p,
+                                                                                   g.diag.p, tg.T.p, tg.dH[nxt].p);
+      cur = nxt;
     }
     CK_LAUNCH();
+    std::vector<double> terms(P);
+    CK(cudaMemcpyAsync(terms.data(), tg.terms.p, terms.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    double loss = 0.0;
+    for (double x : terms) loss += x;
+    loss /= P;
     return loss;
   }
 };
