@@ -34,6 +34,7 @@
 #include "multigrid.h"
 #include "persistent.cuh"
 #include "flex.cuh"
+#include "columns.cuh"
 #include "hybrid_device.cuh"
 #include "generic.cuh"
 #include "observation.cuh"
@@ -1379,6 +1380,21 @@ void ensure_multigrid(DeviceEngine& e) {
   e.mg = build_multigrid(e.n, Lptr, Lcol, Lval, Ld, e.stream, e.stats.h2d_bytes);
 }
 
+// The CMG fallback from the current x after `used` iterations; returns its
+// largest per-column iteration count.
+template <int K>
+int run_fallback(DeviceEngine& e, BlockWork& w, Launch L, int budget, int used, SolveTimings& tm) {
+  tm.fallbacks += 1;
+  ensure_multigrid(e);
+  k_reactivate<K><<<1, 128, 0, L.s>>>(w.s);
+  const int saved = e.preconditioner;
+  e.preconditioner = 2;
+  pcg_restart<K>(e, w, L, false, true);
+  int done = pcg_run_mg<K>(e, w, L, std::max(1, budget - used), tm);
+  e.preconditioner = saved;
+  return done;
+}
+
 // After a capped learned launch: returns -1 when every column converged (the
 // state comes back with the extraction results), else runs the CMG fallback
 // and returns its largest per-column iteration count.
@@ -1389,19 +1405,10 @@ int learned_fallback(DeviceEngine& e, BlockWork& w, Launch L, int budget, SolveT
   CK(cudaMemcpyAsync(&bd, w.s.breakdown, sizeof(int), cudaMemcpyDeviceToHost, L.s));
   CK(cudaStreamSynchronize(L.s));
   if (*e.h_nactive == 0 && bd < 0) return -1;
-  tm.fallbacks += 1;
-  ensure_multigrid(e);
   std::vector<int> it(K);
   CK(cudaMemcpyAsync(it.data(), w.s.iters, K * sizeof(int), cudaMemcpyDeviceToHost, L.s));
   CK(cudaStreamSynchronize(L.s));
-  const int used = *std::max_element(it.begin(), it.end());
-  k_reactivate<K><<<1, 128, 0, L.s>>>(w.s);
-  const int saved = e.preconditioner;
-  e.preconditioner = 2;
-  pcg_restart<K>(e, w, L, false, true);
-  int done = pcg_run_mg<K>(e, w, L, std::max(1, budget - used), tm);
-  e.preconditioner = saved;
-  return done;
+  return run_fallback<K>(e, w, L, budget, *std::max_element(it.begin(), it.end()), tm);
 }
 
 // Segmented firm-side gather (op as in k_seg_firm) finished per row.
@@ -1424,6 +1431,46 @@ void firm_gather(DeviceEngine& e, BlockWork& w, Launch L, const double* coef, co
   CK_LAUNCH();
 }
 
+// The one-block-per-column solve (columns.cuh) serves the Jacobi and the
+// degree-1 forms of Laplacians with at most COL_MAX_VERTICES vertices; as in
+// the cooperative kernels the degree-1 stage takes blocks of 32 or 64 columns.
+template <int K>
+bool column_poly(const DeviceEngine& e) {
+  return flex_width<K>() && (e.preconditioner == 3 || e.preconditioner == 4);
+}
+
+template <int K>
+bool column_form(const DeviceEngine& e) {
+  bool mat;
+  return e.preconditioner != 2 && column_smem(e.n, e.lap_seg.count, e.L_col.n, column_poly<K>(e), &mat) > 0;
+}
+
+template <int K>
+void launch_columns(DeviceEngine& e, BlockWork& w, Launch L, int ncols, double tol, int iterations, bool fresh) {
+  ColumnPcg a{};
+  a.n = e.n;
+  a.nseg = e.lap_seg.count;
+  a.nnz = uint32_t(e.L_col.n);
+  a.K = K;
+  a.seg_begin = e.lap_seg.begin.p;
+  a.seg_end = e.lap_seg.end.p;
+  a.row_first = e.lap_seg.row_first.p;
+  a.col = e.L_col.p;
+  a.val = e.L_val.p;
+  a.diag = e.L_diag.p;
+  a.dinv = e.L_dinv.p;
+  a.wa = e.flex_wa.p;
+  a.ws = e.flex_ws.p;
+  a.b = w.b.p;
+  a.x = w.x.p;
+  a.s = w.s;
+  a.ncols = ncols;
+  a.fresh = fresh ? 1 : 0;
+  a.max_iters = iterations;
+  a.tol = tol;
+  launch_pcg_columns(a, column_poly<K>(e), L.s);
+}
+
 // Solve the K right-hand sides held in w.bW / w.bF (columns >= ncols are zero).
 // On return w.alpha holds the worker solution and w.x[0, F) the firm solution.
 template <int K>
@@ -1432,16 +1479,19 @@ BlockOutcome solve_block(DeviceEngine& e, BlockWork& w, int ncols, const SolveOp
   BlockOutcome out;
   // hybrid RHS (Schur reduction of the worker block) and its column sums
   firm_gather<K, 1, 1>(e, w, L, e.cell_scale.p, w.bW.p, nullptr, 0.0, w.bF.p, w.bW.p, nullptr, w.b.p, e.partial.p);
-  finish(e.partial.p, L.grid, 2 * K, w.tot.p, L.s);
-  k_pcg_init_state<K><<<1, 128, 0, L.s>>>(w.tot.p, ncols, o.pcg_tolerance, double(e.n), w.s);
+  const bool columns = column_form<K>(e);
+  if (!columns) {  // (the column solve forms its own means and tolerances)
+    finish(e.partial.p, L.grid, 2 * K, w.tot.p, L.s);
+    k_pcg_init_state<K><<<1, 128, 0, L.s>>>(w.tot.p, ncols, o.pcg_tolerance, double(e.n), w.s);
+  }
   // blocks of 32 or 64 columns in the mixed-precision or polynomial forms run
   // the single-kernel solve, which forms its own start from x; narrower
   // blocks of those forms run FP64 Jacobi PCG
-  const bool flex = flex_width<K>() && flex_form(e, o);
+  const bool flex = !columns && flex_width<K>() && flex_form(e, o);
   // the multigrid and learned forms and the three-barrier Jacobi kernel take
   // p and r.z from the restart
   const bool directions = e.preconditioner == 2 || !two_barrier_form<K, double>();
-  if (!flex) {
+  if (!flex && !columns) {
     pcg_restart<K>(e, w, L, true, directions);
   }
 
@@ -1455,7 +1505,13 @@ BlockOutcome solve_block(DeviceEngine& e, BlockWork& w, int ncols, const SolveOp
     if (budget <= 0)
       fail(PCG_MAX_ITERATIONS, "pcg", "blocked PCG reached the iteration limit " + std::to_string(o.maximum_iterations));
     int done;
-    if (flex) {
+    const bool learned_cap = columns && column_poly<K>(e) && e.preconditioner == 3;
+    if (columns) {
+      launch_columns<K>(e, w, L, ncols, o.pcg_tolerance, learned_cap ? std::min(budget, LEARNED_CAP) : budget,
+                        ladder == 0);
+      tm.spmm_launches += 1;
+      done = -1;
+    } else if (flex) {
       // like the Jacobi kernel below, the state comes back with the
       // extraction results
       const bool learned = e.preconditioner == 3;
@@ -1477,12 +1533,15 @@ BlockOutcome solve_block(DeviceEngine& e, BlockWork& w, int ncols, const SolveOp
       done = -1;
       tm.spmm_launches += 1;
     }
-    const bool deferred = done < 0;
-    if (!deferred) {
-      total_iters = done;
+    bool deferred = done < 0;
+    auto check_limit = [&] {
       if (*e.h_nactive != 0)
         fail(PCG_MAX_ITERATIONS, "pcg",
              "blocked PCG reached the iteration limit " + std::to_string(o.maximum_iterations));
+    };
+    if (!deferred) {
+      total_iters = done;
+      check_limit();
     }
     // the breakdown flag comes back with the extraction results (one host
     // round trip per pass); nothing below is used before it is checked.  A
@@ -1490,28 +1549,42 @@ BlockOutcome solve_block(DeviceEngine& e, BlockWork& w, int ncols, const SolveOp
     // still runs its extraction kernels, and their outputs are discarded by
     // the fail() after the synchronisation: keep those checks ahead of any
     // use of the extracted values
-    CK(cudaMemcpyAsync(e.h_nactive + 1, w.s.breakdown, sizeof(int), cudaMemcpyDeviceToHost, L.s));
-
-    // extraction and complete residual
-    double* pw = e.partial.p;
-    double* pf = e.partial.p + size_t(L.grid) * 2 * K;
-    k_extract_residual<K><<<L.grid, THREADS, 0, L.s>>>(e.W, e.F, e.worker_ptr.p, e.cell_firm.p, e.cell_weight.p,
-                                                       e.worker_diag.p, e.kept_index.p, w.x.p, w.bW.p, w.alpha.p,
-                                                       pw);
-    firm_gather<K, 2, 2>(e, w, L, e.cell_weight.p, w.alpha.p, nullptr, 0.0, w.bF.p, nullptr, w.x.p, nullptr, pf);
-    finish(pw, L.grid, 2 * K, w.tot.p, L.s);
-    finish(pf, L.grid, 2 * K, w.tot.p + 2 * K, L.s);
     std::vector<double> tot(4 * K);
-    CK(cudaMemcpyAsync(tot.data(), w.tot.p, 4 * K * sizeof(double), cudaMemcpyDeviceToHost, L.s));
-    CK(cudaMemcpyAsync(h_rr.data(), w.s.rr, K * sizeof(double), cudaMemcpyDeviceToHost, L.s));
-    CK(cudaMemcpyAsync(h_bb.data(), w.s.bb, K * sizeof(double), cudaMemcpyDeviceToHost, L.s));
-    CK(cudaMemcpyAsync(h_it.data(), w.s.iters, K * sizeof(int), cudaMemcpyDeviceToHost, L.s));
-    CK(cudaStreamSynchronize(L.s));
+    auto extract = [&] {  // extraction and complete residual
+      double* pw = e.partial.p;
+      double* pf = e.partial.p + size_t(L.grid) * 2 * K;
+      k_extract_residual<K><<<L.grid, THREADS, 0, L.s>>>(e.W, e.F, e.worker_ptr.p, e.cell_firm.p, e.cell_weight.p,
+                                                         e.worker_diag.p, e.kept_index.p, w.x.p, w.bW.p, w.alpha.p,
+                                                         pw);
+      firm_gather<K, 2, 2>(e, w, L, e.cell_weight.p, w.alpha.p, nullptr, 0.0, w.bF.p, nullptr, w.x.p, nullptr, pf);
+      finish(pw, L.grid, 2 * K, w.tot.p, L.s);
+      finish(pf, L.grid, 2 * K, w.tot.p + 2 * K, L.s);
+      if (columns)  // (its flags are per column)
+        CK(cudaMemcpyAsync(h_active.data(), w.s.active, K * sizeof(int), cudaMemcpyDeviceToHost, L.s));
+      else
+        CK(cudaMemcpyAsync(e.h_nactive + 1, w.s.breakdown, sizeof(int), cudaMemcpyDeviceToHost, L.s));
+      CK(cudaMemcpyAsync(tot.data(), w.tot.p, 4 * K * sizeof(double), cudaMemcpyDeviceToHost, L.s));
+      CK(cudaMemcpyAsync(h_rr.data(), w.s.rr, K * sizeof(double), cudaMemcpyDeviceToHost, L.s));
+      CK(cudaMemcpyAsync(h_bb.data(), w.s.bb, K * sizeof(double), cudaMemcpyDeviceToHost, L.s));
+      CK(cudaMemcpyAsync(h_it.data(), w.s.iters, K * sizeof(int), cudaMemcpyDeviceToHost, L.s));
+      CK(cudaStreamSynchronize(L.s));
+    };
+    extract();
+    if (columns) {
+      e.h_nactive[0] = int(std::count(h_active.begin(), h_active.end(), 1));
+      const auto bd = std::find(h_active.begin(), h_active.end(), 2);
+      e.h_nactive[1] = bd == h_active.end() ? -1 : int(bd - h_active.begin());
+      if (learned_cap && (e.h_nactive[0] > 0 || e.h_nactive[1] >= 0)) {
+        total_iters = run_fallback<K>(e, w, L, budget, *std::max_element(h_it.begin(), h_it.end()), tm);
+        check_limit();
+        deferred = false;
+        CK(cudaMemcpyAsync(e.h_nactive + 1, w.s.breakdown, sizeof(int), cudaMemcpyDeviceToHost, L.s));
+        extract();
+      }
+    }
     if (deferred) {
       total_iters = *std::max_element(h_it.begin(), h_it.end());
-      if (*e.h_nactive != 0)
-        fail(PCG_MAX_ITERATIONS, "pcg",
-             "blocked PCG reached the iteration limit " + std::to_string(o.maximum_iterations));
+      check_limit();
     }
     if (const int bd = e.h_nactive[1]; bd >= 0)
       fail(PCG_CURVATURE_BREAKDOWN, "pcg", "nonpositive curvature in column " + std::to_string(bd));
@@ -1542,7 +1615,7 @@ BlockOutcome solve_block(DeviceEngine& e, BlockWork& w, int ncols, const SolveOp
     for (int j = 0; j < K; ++j) tol2[j] = tol * tol * h_bb[j];
     CK(cudaMemcpyAsync(w.s.tol2, tol2.data(), K * sizeof(double), cudaMemcpyHostToDevice, L.s));
     CK(cudaMemcpyAsync(w.s.active, h_active.data(), K * sizeof(int), cudaMemcpyHostToDevice, L.s));
-    if (!flex) pcg_restart<K>(e, w, L, false, directions);
+    if (!flex && !columns) pcg_restart<K>(e, w, L, false, directions);
   }
   out.block_iterations = total_iters;
   tm.pcg_iterations += total_iters;
