@@ -684,7 +684,7 @@ __global__ void k_unit_target_sums(uint32_t units, int q, const uint32_t* __rest
 // side sums the worker and firm columns (linear in u).  partial layout as in
 // k_generic_contract.
 template <int K>
-__global__ void k_generic_contract_units(uint32_t units, int q, const uint32_t* __restrict__ unit_cell,
+__global__ void k_generic_contract_units(uint32_t units, int q, uint32_t chunk, const uint32_t* __restrict__ unit_cell,
                                          const uint32_t* __restrict__ cell_worker,
                                          const uint32_t* __restrict__ cell_firm, const double* __restrict__ sums,
                                          const double* __restrict__ beta /* [QMAX][K] */,
@@ -698,15 +698,15 @@ __global__ void k_generic_contract_units(uint32_t units, int q, const uint32_t* 
   for (int c = 0; c < CPT; ++c) v[0][c] = v[1][c] = 0.0;
   const int c0 = int(threadIdx.x % TPR) * CPT;
   if constexpr (TPR == 32 && CPT == 2) {
-    // one warp per unit: the units' workers and firms are loaded 32 at a time
-    // lane-parallel and broadcast, beta sits in shared memory
+    // one warp per unit: the units' workers and firms are loaded `chunk` (at
+    // most 32) at a time lane-parallel and broadcast, beta sits in shared memory
     __shared__ double sbeta[QMAX][K];
     for (int t = threadIdx.x; t < QMAX * K; t += blockDim.x) sbeta[t / K][t % K] = t / K < q ? beta[t] : 0.0;
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const size_t nwarps = size_t(gridDim.x) * blockDim.x / 32;
-    for (size_t i0 = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32 * 32; i0 < units; i0 += nwarps * 32) {
-      const int cnt = int(units - i0 < 32 ? units - i0 : 32);
+    for (size_t i0 = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32 * chunk; i0 < units; i0 += nwarps * chunk) {
+      const int cnt = int(units - i0 < chunk ? units - i0 : chunk);
       uint32_t my_w = 0, my_f = 0;
       if (lane < cnt) {
         uint32_t cell = unit_cell[i0 + lane];
