@@ -57,6 +57,8 @@ constexpr int FINISH_THREADS = 1024;
 __global__ void __launch_bounds__(FINISH_THREADS) k_finish(const double* __restrict__ partial, int blocks, int width,
                                                            double* __restrict__ out) {
   __shared__ double sm[FINISH_THREADS];
+  partial += size_t(blockIdx.y) * blocks * width;  // one of several partial arrays, one after another
+  out += size_t(blockIdx.y) * width;
   int groups = FINISH_THREADS / FINISH_COLS;
   const int o = blockIdx.x * FINISH_COLS + threadIdx.x % FINISH_COLS, g = threadIdx.x / FINISH_COLS;
   double acc = 0.0;
@@ -87,8 +89,9 @@ __global__ void __launch_bounds__(FINISH_THREADS) k_finish(const double* __restr
   }
 }
 
-void finish(const double* partial, int blocks, int width, double* out, cudaStream_t s) {
-  k_finish<<<(width + FINISH_COLS - 1) / FINISH_COLS, FINISH_THREADS, 0, s>>>(partial, blocks, width, out);
+void finish(const double* partial, int blocks, int width, double* out, cudaStream_t s, int arrays = 1) {
+  k_finish<<<dim3((width + FINISH_COLS - 1) / FINISH_COLS, arrays), FINISH_THREADS, 0, s>>>(partial, blocks, width,
+                                                                                           out);
 }
 
 __global__ void k_raw_atoms(uint64_t count, const uint64_t* __restrict__ entity, const uint64_t* __restrict__ trials,
@@ -181,6 +184,11 @@ __global__ void k_fit_cells(uint32_t cells, const uint32_t* __restrict__ cw, con
     }
   }
   block_reduce_cols<1, 4>(v, partial);
+}
+
+// The fit's target-weighted effect means from the first pass's sums.
+__global__ void k_fit_means(const double* __restrict__ sums, double total, double* __restrict__ means) {
+  if (threadIdx.x < 2) means[threadIdx.x] = sums[threadIdx.x] / total;
 }
 
 // ---------------------------------------------------------------------------
@@ -317,9 +325,9 @@ struct DeviceEngine {
   // leave-observation-out target sums per cell (cells x (1 + q)) and the
   // cell-independent quadratic form sum_r w_r R_r R_r' (q x q, upper triangle)
   DBuf<double> obs_cell_sums, obs_s2;
-  // the fused leave-observation-out target pass: its reduced sums and a
-  // second partial buffer
-  DBuf<double> obs_fused, partial2;
+  // the target blocks' contraction sums, and the second partial buffer of the
+  // fused leave-observation-out target pass
+  DBuf<double> draw_sums, partial2;
   std::vector<double> obs_S2;
   // solve-long buffers
   DBuf<double> moments, unit_out, omega, fitted, fit_alpha, partial, small;
@@ -354,6 +362,7 @@ struct DeviceEngine {
   std::map<int, std::unique_ptr<BlockWork>> work;
   // pinned host scalars
   int* h_nactive = nullptr;
+  double* h_pack = nullptr;  // BlockWork::pack of the last solve
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   ~DeviceEngine();
 };
@@ -370,13 +379,22 @@ int device_tuning(const DeviceEngine& e, int* precision, int* preconditioner, do
   return e.tuned;
 }
 
+// Doubles of BlockWork::pack at width K.
+constexpr size_t pack_size(int K) { return size_t(8) * K + (size_t(K) + 2) + size_t(4) * K; }
+constexpr int PACK_MAX_K = 128;
+
 // Per block-width workspace and the captured PCG iteration graph.
 struct BlockWork {
   int K;
   DBuf<double> bW, bF, b, x, r, z, p, q, alpha, cell_val, unit_atoms, dir, tot, seg_buf, fseg_out;
   DBuf<double> piece2, piece3;  // hub firms' level-2 and level-3 partial sums
-  DBuf<double> st;  // 8 * K doubles of per-column state
-  DBuf<int> ist;    // 2 * K + 2 ints
+  // what a solve hands back, in one piece so one copy brings it to the host:
+  // 8 K doubles of per-column state, 2 K + 4 ints (active, iterations, nactive,
+  // breakdown, replacements, the target balance check), 4 K residual sums
+  DBuf<double> pack;
+  double* st = nullptr;
+  int* ist = nullptr;
+  double* residuals = nullptr;
   PcgState s;
   // mixed precision (flex.cuh): increment of x since the last residual
   // replacement, residual, direction and preconditioned residual
@@ -393,7 +411,7 @@ DeviceEngine::~DeviceEngine() {
   // the buffers go back to the device cache: no queued work may still use them
   if (stream) cudaStreamSynchronize(stream);
   work.clear();
-  if (h_nactive) cudaFreeHost(h_nactive);
+  if (h_pack) cudaFreeHost(h_pack);
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
   if (own_stream && stream) cudaStreamDestroy(stream);
@@ -807,7 +825,8 @@ std::shared_ptr<DeviceEngine> make_device_engine(const Compressed& p, const JlaP
   e->partial.alloc(size_t(grid_blocks()) * QMAX * 128 + 1024);
   e->small.alloc(1024);
   e->error.alloc(2);  // [0] first failing unit << 8 | code, [1] maximum leverage (double bits)
-  CK(cudaMallocHost(&e->h_nactive, sizeof(int) * 16));
+  CK(cudaMallocHost(&e->h_pack, pack_size(PACK_MAX_K) * sizeof(double) + 16 * sizeof(int)));
+  e->h_nactive = reinterpret_cast<int*>(e->h_pack + pack_size(PACK_MAX_K));
   {
     int dev = 0, sms = 0, per = 0;
     CK(cudaGetDevice(&dev));
@@ -946,10 +965,10 @@ BlockWork& get_work(DeviceEngine& e) {
   w->fseg_out.alloc(size_t(e.firm_seg.count) * K);
   w->piece2.alloc(size_t(std::max<uint32_t>(e.firm_pieces.n2, 1)) * K);
   w->piece3.alloc(size_t(std::max<uint32_t>(e.firm_pieces.n3, 1)) * K);
-  w->st.alloc(8 * K);
-  w->ist.alloc(2 * K + 4);
-  double* st = w->st.p;
-  int* ist = w->ist.p;
+  w->pack.alloc(pack_size(K));
+  double* st = w->st = w->pack.p;
+  int* ist = w->ist = reinterpret_cast<int*>(st + 8 * K);
+  w->residuals = st + 8 * K + K + 2;
   w->s = PcgState{st, st + K, st + 2 * K, st + 3 * K, st + 4 * K, st + 5 * K, st + 6 * K,
                   ist, ist + K, ist + 2 * K, ist + 2 * K + 1};
   auto& ref = *w;
@@ -1259,8 +1278,8 @@ void launch_flex_v(DeviceEngine& e, BlockWork& w, Launch L, int iterations, bool
   a.b = w.b.p;
   a.partial = e.partial.p;
   a.s = w.s;
-  a.rr_ref = w.st.p + 7 * K;
-  a.replacements = w.ist.p + 2 * K + 2;
+  a.rr_ref = w.st + 7 * K;
+  a.replacements = w.ist + 2 * K + 2;
   a.max_iters = iterations;
   a.fresh = fresh ? 1 : 0;
   a.replace2 = FLEX_REPLACE * FLEX_REPLACE;
@@ -1482,8 +1501,12 @@ void launch_columns(DeviceEngine& e, BlockWork& w, Launch L, int ncols, double t
 
 // Solve the K right-hand sides held in w.bW / w.bF (columns >= ncols are zero).
 // On return w.alpha holds the worker solution and w.x[0, F) the firm solution.
+// One host round trip: the state, the residual sums and the flags come back in
+// one pinned copy after the extraction.  balance: called with the target
+// balance check's word (k_balance_repair) before the solve's own checks.
 template <int K>
-BlockOutcome solve_block(DeviceEngine& e, BlockWork& w, int ncols, const SolveOptions& o, SolveTimings& tm) {
+BlockOutcome solve_block(DeviceEngine& e, BlockWork& w, int ncols, const SolveOptions& o, SolveTimings& tm,
+                         const std::function<void(int)>* balance = nullptr) {
   Launch L{grid_blocks(), e.stream};
   BlockOutcome out;
   // hybrid RHS (Schur reduction of the worker block) and its column sums
@@ -1527,7 +1550,6 @@ BlockOutcome solve_block(DeviceEngine& e, BlockWork& w, int ncols, const SolveOp
       launch_flex<K>(e, w, L, learned ? std::min(budget, LEARNED_CAP) : budget, ladder == 0, o.precision);
       tm.spmm_launches += 1;
       done = learned ? learned_fallback<K>(e, w, L, budget, tm) : -1;
-      if (done < 0) CK(cudaMemcpyAsync(e.h_nactive, w.s.nactive, sizeof(int), cudaMemcpyDeviceToHost, L.s));
     } else if (e.preconditioner == 2) {
       done = pcg_run_mg<K>(e, w, L, budget, tm);
     } else {
@@ -1538,7 +1560,6 @@ BlockOutcome solve_block(DeviceEngine& e, BlockWork& w, int ncols, const SolveOp
       const void* fn = two_barrier_form<K, double>() ? (const void*)k_pcg_persistent_cg<K>
                                                      : (const void*)k_pcg_persistent<K>;
       CK(cudaLaunchCooperativeKernel(fn, dim3(e.coop_blocks), dim3(PERSIST_THREADS), args, 0, L.s));
-      CK(cudaMemcpyAsync(e.h_nactive, w.s.nactive, sizeof(int), cudaMemcpyDeviceToHost, L.s));
       done = -1;
       tm.spmm_launches += 1;
     }
@@ -1558,25 +1579,26 @@ BlockOutcome solve_block(DeviceEngine& e, BlockWork& w, int ncols, const SolveOp
     // still runs its extraction kernels, and their outputs are discarded by
     // the fail() after the synchronisation: keep those checks ahead of any
     // use of the extracted values
-    std::vector<double> tot(4 * K);
+    const double* pk = e.h_pack;
+    const int* pki = reinterpret_cast<const int*>(pk + 8 * K);
+    const double* tot = pk + 8 * K + K + 2;
     auto extract = [&] {  // extraction and complete residual
       double* pw = e.partial.p;
       double* pf = e.partial.p + size_t(L.grid) * 2 * K;
-      k_extract_residual<K><<<L.grid, THREADS, 0, L.s>>>(e.W, e.F, warp_chunk(e.W, L.grid), e.worker_ptr.p, e.cell_firm.p, e.cell_weight.p,
-                                                         e.worker_diag.p, e.kept_index.p, w.x.p, w.bW.p, w.alpha.p,
-                                                         pw);
+      k_extract_residual<K><<<L.grid, THREADS, 0, L.s>>>(e.W, e.F, warp_chunk(e.W, L.grid), e.worker_ptr.p,
+                                                         e.cell_firm.p, e.cell_weight.p, e.worker_diag.p,
+                                                         e.kept_index.p, w.x.p, w.bW.p, w.alpha.p, pw);
       firm_gather<K, 2, 2>(e, w, L, e.cell_weight.p, w.alpha.p, nullptr, 0.0, w.bF.p, nullptr, w.x.p, nullptr, pf);
-      finish(pw, L.grid, 2 * K, w.tot.p, L.s);
-      finish(pf, L.grid, 2 * K, w.tot.p + 2 * K, L.s);
-      if (columns)  // (its flags are per column)
-        CK(cudaMemcpyAsync(h_active.data(), w.s.active, K * sizeof(int), cudaMemcpyDeviceToHost, L.s));
-      else
-        CK(cudaMemcpyAsync(e.h_nactive + 1, w.s.breakdown, sizeof(int), cudaMemcpyDeviceToHost, L.s));
-      CK(cudaMemcpyAsync(tot.data(), w.tot.p, 4 * K * sizeof(double), cudaMemcpyDeviceToHost, L.s));
-      CK(cudaMemcpyAsync(h_rr.data(), w.s.rr, K * sizeof(double), cudaMemcpyDeviceToHost, L.s));
-      CK(cudaMemcpyAsync(h_bb.data(), w.s.bb, K * sizeof(double), cudaMemcpyDeviceToHost, L.s));
-      CK(cudaMemcpyAsync(h_it.data(), w.s.iters, K * sizeof(int), cudaMemcpyDeviceToHost, L.s));
+      finish(pw, L.grid, 2 * K, w.residuals, L.s, 2);
+      CK(cudaMemcpyAsync(e.h_pack, w.pack.p, pack_size(K) * sizeof(double), cudaMemcpyDeviceToHost, L.s));
       CK(cudaStreamSynchronize(L.s));
+      if (balance) (*balance)(pki[2 * K + 3]);
+      std::copy_n(pk + K, K, h_rr.begin());
+      std::copy_n(pk + 2 * K, K, h_bb.begin());
+      std::copy_n(pki, K, h_active.begin());
+      std::copy_n(pki + K, K, h_it.begin());
+      if (deferred) e.h_nactive[0] = pki[2 * K];
+      e.h_nactive[1] = pki[2 * K + 1];
     };
     extract();
     if (columns) {
@@ -1587,7 +1609,6 @@ BlockOutcome solve_block(DeviceEngine& e, BlockWork& w, int ncols, const SolveOp
         total_iters = run_fallback<K>(e, w, L, budget, *std::max_element(h_it.begin(), h_it.end()), tm);
         check_limit();
         deferred = false;
-        CK(cudaMemcpyAsync(e.h_nactive + 1, w.s.breakdown, sizeof(int), cudaMemcpyDeviceToHost, L.s));
         extract();
       }
     }
@@ -1642,6 +1663,57 @@ Components finish_accounting(double w, double f, double c, double t, const char*
   if (std::fabs(t - implied) > 1e-11 * scale)
     fail(ACCOUNTING_IDENTITY_FAILED, phase, "total component differs from worker + firm + 2 covariance");
   return r;
+}
+
+// The target right-hand sides' compatibility repair (reference
+// `balance_score_with_interrupt`, engine.rs:2812-2846): the last worker / firm
+// entry of a column becomes minus the sum of the others (the partials pw, pf).
+// A column 2j is probe j's worker side, 2j + 1 its firm side; ref = sum |d| +
+// |sum d| scales the roundoff gate.  flag: the first failing column, 2 q for
+// an invalid scale, 2 q + 1 for a repair beyond roundoff, else BALANCE_OK.
+constexpr int BALANCE_OK = 0x7fffffff;
+template <int K>
+__global__ void __launch_bounds__(STEP_THREADS) k_balance_repair(const double* __restrict__ pw,
+                                                                 const double* __restrict__ pf, int blocks,
+                                                                 const double* __restrict__ tot, int np,
+                                                                 double* __restrict__ lastW,
+                                                                 double* __restrict__ lastF, int* __restrict__ flag) {
+  constexpr int H = K / 2;
+  __shared__ double sw[K], sf[K], scratch[STEP_THREADS];
+  __shared__ int bad;
+  if (threadIdx.x == 0) bad = BALANCE_OK;
+  redundant_finish<1, K>(pw, blocks, sw, scratch);
+  redundant_finish<1, K>(pf, blocks, sf, scratch);
+  for (int q = threadIdx.x; q < K; q += blockDim.x) {
+    const int j = q / 2;
+    if (j >= np) {
+      lastW[q] = 0.0;
+      lastF[q] = 0.0;
+      continue;
+    }
+    const double ref = tot[H + j] + fabs(tot[j]);
+    if (!isfinite(ref) || ref < 0.0) atomicMin(&bad, 2 * q);
+    const double gate = 4096.0 * 2.220446049250313e-16 * ref;
+    double* last = q & 1 ? lastF + q : lastW + q;
+    const double repaired = q & 1 ? -sf[q] : -sw[q];
+    if ((ref == 0.0 && repaired != *last) || (ref > 0.0 && fabs(repaired - *last) > gate)) atomicMin(&bad, 2 * q + 1);
+    *last = repaired;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) *flag = bad;
+}
+
+// beta[k][j] = -sum_l Sinv[k][l] t[l][j] (k < q; zero beyond): the control
+// coefficients of the full-model solves.
+template <int K>
+__global__ void k_solve_beta(int q, SmallMatrix sinv, const double* __restrict__ t, double* __restrict__ beta) {
+  for (int i = threadIdx.x; i < QMAX * K; i += blockDim.x) {
+    const int k = i / K, j = i % K;
+    double v = 0.0;
+    if (k < q)
+      for (int l = 0; l < q; ++l) v -= sinv.m[k * QMAX + l] * t[l * K + j];
+    beta[i] = v;
+  }
 }
 
 // Leverage right-hand sides of probes [first, first + ncols): Counter-V1
@@ -1783,53 +1855,46 @@ void run_target(DeviceEngine& e, const SolveOptions& o, SolveResult& res, double
   PhiloxKey key = philox_key(o.seed);
   double invT = 1.0 / e.target_total;
   if (res.target_draws.size() != o.probes) res.target_draws.assign(o.probes, Components{});
-  std::vector<double> tot(2 * K), sums(2 * K), draws(3 * K);
   const uint32_t end = o.probe_end ? o.probe_end : o.probes;
+  // every block's contraction sums stay on the device until the last block:
+  // (u^2, v^2, u v) of the compressed engine, the two sides and their total of
+  // the match units with controls, or the fused leave-observation-out sums
+  const size_t slot = e.observation ? size_t(2) * (QMAX + 1) * K : e.generic ? size_t(2) * K : size_t(3) * K;
+  const size_t blocks = o.probe_begin < end ? (end - o.probe_begin + H - 1) / H : 0;
+  if (e.draw_sums.n < slot * blocks) e.draw_sums.alloc(slot * blocks);
+  std::vector<BlockOutcome> outcomes;
+  SmallMatrix sinv{};
+  for (int k = 0; k < e.qa; ++k)
+    for (int l = 0; l < e.qa; ++l) sinv.m[k * QMAX + l] = e.Sinv[k * e.qa + l];
   for (uint32_t first = o.probe_begin; first < end; first += H) {
     int np = int(std::min<uint32_t>(H, end - first));
+    double* sums = e.draw_sums.p + outcomes.size() * slot;
     k_target_direction<H><<<L.grid, THREADS, 0, L.s>>>(e.C, e.tgt_ptr.p, e.tgt_rank.p, e.tgt_count.p,
                                                        e.tgt_scale.p, key, first, np, w.dir.p);
     // direction totals: sum_c d and the reference scale sum_c |d| + |sum_c d|
     k_colsum_abs<H><<<L.grid, THREADS, 0, L.s>>>(e.C, w.dir.p, e.partial.p);
     finish(e.partial.p, L.grid, 2 * H, w.tot.p, L.s);
-    CK(cudaMemcpyAsync(tot.data(), w.tot.p, 2 * H * sizeof(double), cudaMemcpyDeviceToHost, L.s));
     k_target_scores<K><<<L.grid, THREADS, 0, L.s>>>(e.W, 0, e.worker_ptr.p, nullptr, w.dir.p, e.cell_target.p, invT,
                                                     w.tot.p, w.bW.p);
     firm_gather<K, 3, 0>(e, w, L, e.cell_target.p, w.dir.p, w.tot.p, invT, nullptr, nullptr, nullptr, w.bF.p, nullptr);
-    // balance repair (reference `balance_score_with_interrupt`, engine.rs:2812-2846):
-    // the last worker / firm entry becomes minus the sum of the others
+    double* pf = e.partial.p + size_t(L.grid) * K;
     k_colsum<K><<<L.grid, THREADS, 0, L.s>>>(e.W - 1, w.bW.p, e.partial.p);
-    finish(e.partial.p, L.grid, K, w.tot.p + 2 * K, L.s);
-    k_colsum<K><<<L.grid, THREADS, 0, L.s>>>(e.F - 1, w.bF.p, e.partial.p);
-    finish(e.partial.p, L.grid, K, w.tot.p + 3 * K, L.s);
-    std::vector<double> lastW(K), lastF(K), pre(2 * K);
-    CK(cudaMemcpyAsync(pre.data(), w.tot.p + 2 * K, 2 * K * sizeof(double), cudaMemcpyDeviceToHost, L.s));
-    CK(cudaMemcpyAsync(lastW.data(), w.bW.p + size_t(e.W - 1) * K, K * sizeof(double), cudaMemcpyDeviceToHost, L.s));
-    CK(cudaMemcpyAsync(lastF.data(), w.bF.p + size_t(e.F - 1) * K, K * sizeof(double), cudaMemcpyDeviceToHost, L.s));
-    CK(cudaStreamSynchronize(L.s));
-    for (int q = 0; q < K; ++q) {
-      int j = q / 2;
-      if (j >= np) {
-        lastW[q] = 0.0;
-        lastF[q] = 0.0;
-        continue;
-      }
-      double ref = tot[H + j] + std::fabs(tot[j]);
-      if (!std::isfinite(ref) || ref < 0.0)
+    k_colsum<K><<<L.grid, THREADS, 0, L.s>>>(e.F - 1, w.bF.p, pf);
+    k_balance_repair<K><<<1, STEP_THREADS, 0, L.s>>>(e.partial.p, pf, L.grid, w.tot.p, np,
+                                                     w.bW.p + size_t(e.W - 1) * K, w.bF.p + size_t(e.F - 1) * K,
+                                                     w.ist + 2 * K + 3);
+    CK_LAUNCH();
+    const std::function<void(int)> balance = [&](int flag) {
+      if (flag == BALANCE_OK) return;
+      const int q = flag / 2;
+      const std::string probe = std::to_string(first + q / 2);
+      if (flag % 2 == 0)
         fail(TARGET_CENTERING_FAILED, "jla_target",
-             "target reference scale is invalid at probe " + std::to_string(first + j) + ", side centered");
-      double gate = 4096.0 * 2.220446049250313e-16 * ref;
-      double& last = (q & 1) ? lastF[q] : lastW[q];
-      double repaired = (q & 1) ? -pre[K + q] : -pre[q];
-      if ((ref == 0.0 && repaired != last) || (ref > 0.0 && std::fabs(repaired - last) > gate))
-        fail(TARGET_CENTERING_FAILED, "jla_target",
-             "compatibility repair exceeded roundoff at probe " + std::to_string(first + j) +
-                 ((q & 1) ? ", side Firm" : ", side Worker"));
-      last = repaired;
-    }
-    CK(cudaMemcpyAsync(w.bW.p + size_t(e.W - 1) * K, lastW.data(), K * sizeof(double), cudaMemcpyHostToDevice, L.s));
-    CK(cudaMemcpyAsync(w.bF.p + size_t(e.F - 1) * K, lastF.data(), K * sizeof(double), cudaMemcpyHostToDevice, L.s));
-    BlockOutcome bo = solve_block<K>(e, w, 2 * np, o, res.timings);
+             "target reference scale is invalid at probe " + probe + ", side centered");
+      fail(TARGET_CENTERING_FAILED, "jla_target",
+           "compatibility repair exceeded roundoff at probe " + probe + ((q & 1) ? ", side Firm" : ", side Worker"));
+    };
+    outcomes.push_back(solve_block<K>(e, w, 2 * np, o, res.timings, &balance));
     if (!e.generic) {
       if (o.numerical)  // the contraction plus the cells' target fold sums of the attachment
         k_contract_folds<K><<<L.grid, THREADS, 0, L.s>>>(e.C, e.cell_worker.p, e.cell_firm.p, e.omega.p, w.alpha.p,
@@ -1837,41 +1902,69 @@ void run_target(DeviceEngine& e, const SolveOptions& o, SolveResult& res, double
       else
         k_contract<K><<<L.grid, THREADS, 0, L.s>>>(e.C, e.cell_worker.p, e.cell_firm.p, e.omega.p, w.alpha.p, w.x.p,
                                                    e.partial.p);
-      finish(e.partial.p, L.grid, 3 * K, w.tot.p, L.s);
-      CK(cudaMemcpyAsync(draws.data(), w.tot.p, 3 * K * sizeof(double), cudaMemcpyDeviceToHost, L.s));
-      CK(cudaStreamSynchronize(L.s));
+      finish(e.partial.p, L.grid, 3 * K, sums, L.s);
+    } else if (e.observation) {
+      // one pass over the cells: the control sums and the draws' beta-free parts
+      if (!e.partial2.p) e.partial2.alloc(size_t(L.grid) * (QMAX + 1) * 128 + 1024);
+      k_obs_target_cells<K><<<L.grid, THREADS, 0, L.s>>>(e.C, e.qa, e.cell_worker.p, e.cell_firm.p,
+                                                         e.qa > 0 ? e.cellQ.p : nullptr, e.obs_cell_sums.p,
+                                                         w.alpha.p, w.x.p, e.partial.p, e.partial2.p);
+      finish(e.partial.p, L.grid, (QMAX + 1) * K, sums, L.s);
+      finish(e.partial2.p, L.grid, (QMAX + 1) * K, sums + (QMAX + 1) * K, L.s);
+      if (o.numerical) {  // the attachment's per-row target folds of this block
+        k_solve_beta<K><<<1, 512, 0, L.s>>>(e.qa, sinv, sums, e.beta_buf.p);
+        k_obs_num_folds<K><<<L.grid, THREADS, 0, L.s>>>(e.C, e.qa, uint64_t(first), np, e.unit_ptr.p,
+                                                        e.cell_rows.p, e.cell_worker.p, e.cell_firm.p, w.alpha.p,
+                                                        w.x.p, e.beta_buf.p, e.Rd.p, e.y_work, y_center,
+                                                        e.residual.p, double((o.probes + 1) / 2),
+                                                        double(o.probes / 2), e.num_row_fold.p);
+      }
     } else {
       // full-model solves: beta = -S^{-1} Q'W X theta_fe per column, then the
       // row-level contraction over match groups
-      std::vector<double> t(QMAX * K, 0.0), beta(QMAX * K, 0.0), g2(2 * K, 0.0);
-      auto solve_beta = [&] {
+      if (e.qa > 0) {
+        k_target_control_cells<K><<<L.grid, THREADS, 0, L.s>>>(e.C, e.qa, e.cell_worker.p, e.cell_firm.p,
+                                                               e.cellQ.p, w.alpha.p, w.x.p, e.partial.p);
+        finish(e.partial.p, L.grid, QMAX * K, w.tot.p, L.s);
+      }
+      k_solve_beta<K><<<1, 512, 0, L.s>>>(e.qa, sinv, w.tot.p, e.beta_buf.p);
+      k_generic_contract_units<K><<<L.grid, THREADS, 0, L.s>>>(e.G, e.qa, warp_chunk(e.G, L.grid), e.unit_cell.p,
+                                                               e.cell_worker.p, e.cell_firm.p, e.unit_sums.p,
+                                                               e.beta_buf.p, w.alpha.p, w.x.p, e.partial.p);
+      if (o.numerical)  // the attachment's match-unit target folds of this block
+        k_num_block_folds<K><<<L.grid, THREADS, 0, L.s>>>(e.G, e.qa, uint64_t(first), np, e.unit_cell.p,
+                                                          e.cell_worker.p, e.cell_firm.p, w.alpha.p, w.x.p,
+                                                          e.beta_buf.p, e.num_block_sums.p,
+                                                          double((o.probes + 1) / 2), double(o.probes / 2),
+                                                          e.num_unit_fold.p);
+      finish(e.partial.p, L.grid, 2 * K, sums, L.s);
+    }
+    CK_LAUNCH();
+  }
+  // the draws of every block
+  std::vector<double> all(slot * outcomes.size()), beta(QMAX * K, 0.0), draws(3 * K), g2(2 * K);
+  if (!all.empty())
+    CK(cudaMemcpyAsync(all.data(), e.draw_sums.p, all.size() * sizeof(double), cudaMemcpyDeviceToHost, L.s));
+  CK(cudaStreamSynchronize(L.s));
+  for (size_t blk = 0; blk < outcomes.size(); ++blk) {
+    const uint32_t first = o.probe_begin + uint32_t(blk) * H;
+    const int np = int(std::min<uint32_t>(H, end - first));
+    const BlockOutcome& bo = outcomes[blk];
+    const double* f = all.data() + blk * slot;
+    if (!e.generic) {
+      std::copy_n(f, 3 * K, draws.begin());
+    } else {
+      std::copy_n(f, std::min<size_t>(slot, 2 * K), g2.begin());
+      if (e.observation) {
+        const double* A = f + QMAX * K;
+        const double* B = f + (QMAX + 1) * K;
+        const double* Atot = f + (2 * QMAX + 1) * K;
         for (int k = 0; k < e.qa; ++k)
           for (int j = 0; j < K; ++j) {
             double v = 0.0;
-            for (int l = 0; l < e.qa; ++l) v -= e.Sinv[k * e.qa + l] * t[l * K + j];
+            for (int l = 0; l < e.qa; ++l) v -= e.Sinv[k * e.qa + l] * f[l * K + j];
             beta[k * K + j] = v;
           }
-      };
-      if (e.observation) {
-        // one pass over the cells: the control sums and the draws' beta-free parts
-        if (!e.obs_fused.p) {
-          e.obs_fused.alloc(2 * (QMAX + 1) * 128);
-          e.partial2.alloc(size_t(L.grid) * (QMAX + 1) * 128 + 1024);
-        }
-        k_obs_target_cells<K><<<L.grid, THREADS, 0, L.s>>>(e.C, e.qa, e.cell_worker.p, e.cell_firm.p,
-                                                           e.qa > 0 ? e.cellQ.p : nullptr, e.obs_cell_sums.p,
-                                                           w.alpha.p, w.x.p, e.partial.p, e.partial2.p);
-        finish(e.partial.p, L.grid, (QMAX + 1) * K, e.obs_fused.p, L.s);
-        finish(e.partial2.p, L.grid, (QMAX + 1) * K, e.obs_fused.p + (QMAX + 1) * K, L.s);
-        std::vector<double> f(2 * (QMAX + 1) * K);
-        CK(cudaMemcpyAsync(f.data(), e.obs_fused.p, f.size() * sizeof(double), cudaMemcpyDeviceToHost, L.s));
-        CK(cudaStreamSynchronize(L.s));
-        const double* A = f.data() + QMAX * K;
-        const double* B = f.data() + (QMAX + 1) * K;
-        const double* Atot = f.data() + (2 * QMAX + 1) * K;
-        for (int k = 0; k < e.qa; ++k)
-          for (int j = 0; j < K; ++j) t[k * K + j] = f[k * K + j];
-        solve_beta();
         for (int j = 0; j < K; ++j) {
           double v = A[j];
           for (int k = 0; k < e.qa; ++k) v += 2.0 * B[k * K + j] * beta[k * K + j];
@@ -1883,36 +1976,6 @@ void run_target(DeviceEngine& e, const SolveOptions& o, SolveResult& res, double
             v += 2.0 * (B[k * K + j] + B[k * K + j + 1]) * (beta[k * K + j] + beta[k * K + j + 1]);
           g2[K + j] = v;
         }
-        if (o.numerical) {  // the attachment's per-row target folds of this block
-          CK(cudaMemcpyAsync(e.beta_buf.p, beta.data(), QMAX * K * sizeof(double), cudaMemcpyHostToDevice, L.s));
-          k_obs_num_folds<K><<<L.grid, THREADS, 0, L.s>>>(e.C, e.qa, uint64_t(first), np, e.unit_ptr.p,
-                                                          e.cell_rows.p, e.cell_worker.p, e.cell_firm.p, w.alpha.p,
-                                                          w.x.p, e.beta_buf.p, e.Rd.p, e.y_work, y_center,
-                                                          e.residual.p, double((o.probes + 1) / 2),
-                                                          double(o.probes / 2), e.num_row_fold.p);
-        }
-      } else {
-        if (e.qa > 0) {
-          k_target_control_cells<K><<<L.grid, THREADS, 0, L.s>>>(e.C, e.qa, e.cell_worker.p, e.cell_firm.p,
-                                                                 e.cellQ.p, w.alpha.p, w.x.p, e.partial.p);
-          finish(e.partial.p, L.grid, QMAX * K, w.tot.p, L.s);
-          CK(cudaMemcpyAsync(t.data(), w.tot.p, QMAX * K * sizeof(double), cudaMemcpyDeviceToHost, L.s));
-          CK(cudaStreamSynchronize(L.s));
-        }
-        solve_beta();
-        CK(cudaMemcpyAsync(e.beta_buf.p, beta.data(), QMAX * K * sizeof(double), cudaMemcpyHostToDevice, L.s));
-        k_generic_contract_units<K><<<L.grid, THREADS, 0, L.s>>>(e.G, e.qa, warp_chunk(e.G, L.grid), e.unit_cell.p, e.cell_worker.p,
-                                                                 e.cell_firm.p, e.unit_sums.p, e.beta_buf.p,
-                                                                 w.alpha.p, w.x.p, e.partial.p);
-        if (o.numerical)  // the attachment's match-unit target folds of this block
-          k_num_block_folds<K><<<L.grid, THREADS, 0, L.s>>>(e.G, e.qa, uint64_t(first), np, e.unit_cell.p,
-                                                            e.cell_worker.p, e.cell_firm.p, w.alpha.p, w.x.p,
-                                                            e.beta_buf.p, e.num_block_sums.p,
-                                                            double((o.probes + 1) / 2), double(o.probes / 2),
-                                                            e.num_unit_fold.p);
-        finish(e.partial.p, L.grid, 2 * K, w.tot.p, L.s);
-        CK(cudaMemcpyAsync(g2.data(), w.tot.p, 2 * K * sizeof(double), cudaMemcpyDeviceToHost, L.s));
-        CK(cudaStreamSynchronize(L.s));
       }
       if (e.observation && e.qa > 0) {
         // the cell-independent beta' S2 beta terms of every column and of the total
@@ -2078,11 +2141,18 @@ void shard_upload(DeviceEngine& e, const double* in) {
 // the leverage-adjustment kernel fed with exact moments (projection n_g h_c,
 // residual 1 - n_g h_c, no Monte Carlo bias or variance).
 
+// One-hot right-hand sides of the block's cells, the previous block's taken
+// back (by the same thread: a column's old and new entry may coincide).
 template <int K>
 __global__ void k_exact_rhs(uint32_t first, int ncols, const uint32_t* __restrict__ cw,
                             const uint32_t* __restrict__ cf, double* __restrict__ bW, double* __restrict__ bF) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < ncols; j += gridDim.x * blockDim.x) {
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < K; j += gridDim.x * blockDim.x) {
     const uint32_t c = first + uint32_t(j);
+    if (first >= uint32_t(K)) {
+      bW[size_t(cw[c - K]) * K + j] = 0.0;
+      bF[size_t(cf[c - K]) * K + j] = 0.0;
+    }
+    if (j >= ncols) continue;
     bW[size_t(cw[c]) * K + j] = 1.0;
     bF[size_t(cf[c]) * K + j] = 1.0;
   }
@@ -2173,25 +2243,32 @@ void run_exact(DeviceEngine& e, const Compressed& p, const SolveOptions& o, Solv
   k_gather<1><<<L.grid, THREADS, 0, L.s>>>(e.F, e.firm_ptr.p, e.firm_cells.p, cmass.p, fshare.p);
   SolveOptions oe = o;
   oe.pcg_tolerance = std::min(o.pcg_tolerance, 1e-10);
-  std::vector<double> B(size_t(e.C) * 3), sums(5 * K);
+  std::vector<double> B(size_t(e.C) * 3);
+  const size_t blocks = (size_t(e.C) + K - 1) / K;
+  DBuf<double> block_sums(blocks * 5 * K);  // read once, after the last block
+  CK(cudaMemsetAsync(w.bW.p, 0, w.bW.bytes(), L.s));
+  CK(cudaMemsetAsync(w.bF.p, 0, w.bF.bytes(), L.s));
   for (uint32_t first = 0; first < e.C; first += K) {
     const int ncols = int(std::min<uint32_t>(K, e.C - first));
-    CK(cudaMemsetAsync(w.bW.p, 0, w.bW.bytes(), L.s));
-    CK(cudaMemsetAsync(w.bF.p, 0, w.bF.bytes(), L.s));
     k_exact_rhs<K><<<1, 128, 0, L.s>>>(first, ncols, e.cell_worker.p, e.cell_firm.p, w.bW.p, w.bF.p);
     CK_LAUNCH();
     solve_block<K>(e, w, ncols, oe, res.timings);
     k_exact_sums<K><<<L.grid, THREADS, 0, L.s>>>(e.W, e.F, e.C, wshare.p, fshare.p, cmass.p, e.cell_worker.p,
                                                  e.cell_firm.p, w.alpha.p, w.x.p, e.partial.p);
-    finish(e.partial.p, L.grid, 5 * K, w.tot.p, L.s);
+    finish(e.partial.p, L.grid, 5 * K, block_sums.p + size_t(first) * 5, L.s);
     k_exact_moments<K><<<1, 128, 0, L.s>>>(first, ncols, e.cell_worker.p, e.cell_firm.p, w.alpha.p, w.x.p,
                                            e.unit_ptr.p, e.unit_count_f.p, e.moments.p);
-    CK(cudaMemcpyAsync(sums.data(), w.tot.p, 5 * K * sizeof(double), cudaMemcpyDeviceToHost, L.s));
+  }
+  {
+    std::vector<double> all(blocks * 5 * K);
+    CK(cudaMemcpyAsync(all.data(), block_sums.p, all.size() * sizeof(double), cudaMemcpyDeviceToHost, L.s));
     CK(cudaStreamSynchronize(L.s));
-    for (int j = 0; j < ncols; ++j) {
+    for (size_t c = 0; c < e.C; ++c) {
+      const double* sums = all.data() + c / K * 5 * K;
+      const int j = int(c % K);
       const double aw = sums[j], aw2 = sums[K + j], pf = sums[2 * K + j], pf2 = sums[3 * K + j],
                    x = sums[4 * K + j];
-      double* b = &B[size_t(first + j) * 3];
+      double* b = &B[c * 3];
       b[0] = aw2 - aw * aw;
       b[1] = pf2 - pf * pf;
       b[2] = x - aw * pf;
@@ -2403,18 +2480,15 @@ void run_jla(DeviceEngine& e, const Compressed& p, const JlaPlan& plan, const So
     k_fit_cells<<<L.grid, THREADS, 0, L.s>>>(e.C, e.cell_worker.p, e.cell_firm.p, w.alpha.p, w.x.p, e.cell_target.p,
                                              e.fitted.p, 0, nullptr, e.partial.p);
     finish(e.partial.p, L.grid, 4, e.small.p, L.s);
-    std::vector<double> m(4);
-    CK(cudaMemcpyAsync(m.data(), e.small.p, 4 * sizeof(double), cudaMemcpyDeviceToHost, L.s));
-    CK(cudaStreamSynchronize(L.s));
-    double means[2] = {m[0] / p.target_total, m[1] / p.target_total};
-    if (!std::isfinite(means[0]) || !std::isfinite(means[1]))
-      fail(CORRECTION_NONFINITE, "jla_plugin", "centered effect mean is nonfinite");
-    CK(cudaMemcpyAsync(e.small.p + 8, means, 2 * sizeof(double), cudaMemcpyHostToDevice, L.s));
+    k_fit_means<<<1, 32, 0, L.s>>>(e.small.p, p.target_total, e.small.p + 4);
     k_fit_cells<<<L.grid, THREADS, 0, L.s>>>(e.C, e.cell_worker.p, e.cell_firm.p, w.alpha.p, w.x.p, e.cell_target.p,
-                                             e.fitted.p, 1, e.small.p + 8, e.partial.p);
+                                             e.fitted.p, 1, e.small.p + 4, e.partial.p);
     finish(e.partial.p, L.grid, 4, e.small.p, L.s);
-    CK(cudaMemcpyAsync(m.data(), e.small.p, 4 * sizeof(double), cudaMemcpyDeviceToHost, L.s));
+    std::vector<double> m(6);
+    CK(cudaMemcpyAsync(m.data(), e.small.p, 6 * sizeof(double), cudaMemcpyDeviceToHost, L.s));
     CK(cudaStreamSynchronize(L.s));
+    if (!std::isfinite(m[4]) || !std::isfinite(m[5]))
+      fail(CORRECTION_NONFINITE, "jla_plugin", "centered effect mean is nonfinite");
     double T = p.target_total;
     res.plugin = finish_accounting(m[0] / T, m[1] / T, m[2] / T, m[3] / T, "jla_components");
     e.shard_plugin = res.plugin;
@@ -2733,14 +2807,11 @@ void run_generic(DeviceEngine& e, const Compressed& p, const JlaPlan& plan, cons
       k_fit_cells<<<L.grid, THREADS, 0, L.s>>>(e.C, e.cell_worker.p, e.cell_firm.p, w.alpha.p, w.x.p, e.cell_target.p,
                                                e.fitted.p, 0, nullptr, e.partial.p);
       finish(e.partial.p, L.grid, 4, e.small.p, L.s);
-      std::vector<double> m(4);
-      CK(cudaMemcpyAsync(m.data(), e.small.p, 4 * sizeof(double), cudaMemcpyDeviceToHost, L.s));
-      CK(cudaStreamSynchronize(L.s));
-      double means[2] = {m[0] / p.target_total, m[1] / p.target_total};
-      CK(cudaMemcpyAsync(e.small.p + 8, means, 2 * sizeof(double), cudaMemcpyHostToDevice, L.s));
+      k_fit_means<<<1, 32, 0, L.s>>>(e.small.p, p.target_total, e.small.p + 4);
       k_fit_cells<<<L.grid, THREADS, 0, L.s>>>(e.C, e.cell_worker.p, e.cell_firm.p, w.alpha.p, w.x.p, e.cell_target.p,
-                                               e.fitted.p, 1, e.small.p + 8, e.partial.p);
+                                               e.fitted.p, 1, e.small.p + 4, e.partial.p);
       finish(e.partial.p, L.grid, 4, e.small.p, L.s);
+      std::vector<double> m(4);
       CK(cudaMemcpyAsync(m.data(), e.small.p, 4 * sizeof(double), cudaMemcpyDeviceToHost, L.s));
       CK(cudaStreamSynchronize(L.s));
       double T = p.target_total;
@@ -3092,7 +3163,7 @@ void kernel_benchmark_k(DeviceEngine& e, int kernel, int launches, double* ms, d
                                                           e.flex_valw.p);
       CK_LAUNCH();
     }
-    CK(cudaMemsetAsync(w.ist.p + 2 * K + 2, 0, sizeof(int), L.s));
+    CK(cudaMemsetAsync(w.ist + 2 * K + 2, 0, sizeof(int), L.s));
   }
   std::vector<float> times;
   for (int i = 0; i < launches; ++i) {
@@ -3183,7 +3254,7 @@ void kernel_benchmark_k(DeviceEngine& e, int kernel, int launches, double* ms, d
     // replacements of an average launch: x and xi read and written, x
     // gathered, FP64 segment products written and read, b and x read, r written
     int reps = 0;
-    CK(cudaMemcpy(&reps, w.ist.p + 2 * K + 2, sizeof(int), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(&reps, w.ist + 2 * K + 2, sizeof(int), cudaMemcpyDeviceToHost));
     const double per_launch = double(reps) / launches;
     *bytes += n * K * (8.0 + 4 + 8 + 4 + 4 + 4) +
               per_launch * (nnz * 12 + nseg * 16 + n * 16 + n * K * 52.0 + 16 * nseg * K);
