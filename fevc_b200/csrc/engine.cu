@@ -233,6 +233,7 @@ int device_count() {
   return n;
 }
 
+// Blocks of the streaming kernels at most: the size the partial buffers have.
 static int grid_blocks() {
   static int blocks = 0;
   if (!blocks) {
@@ -298,8 +299,13 @@ struct DeviceEngine {
   int tune_precision[3] = {0, 0, 0}, tune_preconditioner[3] = {0, 0, 0};
   double tune_ms[3] = {0.0, 0.0, 0.0};
   Segments lap_seg, firm_seg;
-  PieceLevels firm_pieces;  // hierarchical finish of the hub firms' segment sums
+  HubRows firm_hubs;  // firms of many segments, summed by a block each
   int coop_blocks = 0;
+  // blocks of the streaming kernels: eight warps each, one warp for every
+  // worker, cell or vertex of the problem, at least two blocks an SM and at
+  // most grid_blocks().  A reduction's finish reads one partial per block:
+  // 7.5 us for 1,184 of them (128 columns), 3.5 us for 296
+  int grid = 0;
   std::vector<RhsReceipt> control_receipts;  // the control projections' solves (generic estimator)
   // generic (controlled) estimator: row-level data and the control geometry
   bool generic = false;
@@ -387,7 +393,7 @@ constexpr int PACK_MAX_K = 128;
 struct BlockWork {
   int K;
   DBuf<double> bW, bF, b, x, r, z, p, q, alpha, cell_val, unit_atoms, dir, tot, seg_buf, fseg_out;
-  DBuf<double> piece2, piece3;  // hub firms' level-2 and level-3 partial sums
+  DBuf<double> hub_sums;  // the hub firms' sums
   // what a solve hands back, in one piece so one copy brings it to the host:
   // 8 K doubles of per-column state, 2 K + 4 ints (active, iterations, nactive,
   // breakdown, replacements, the target balance check), 4 K residual sums
@@ -499,6 +505,9 @@ std::shared_ptr<DeviceEngine> make_device_engine(const Compressed& p, const JlaP
   e->G = uint32_t(plan.del_cell.size());
   e->S = uint32_t(plan.tgt_cell.size());
   e->target_total = p.target_total;
+  const size_t items = std::max({size_t(e->W), size_t(e->C), size_t(e->F), size_t(e->G)});
+  const size_t most = size_t(grid_blocks());
+  e->grid = int(std::min(most, std::max(most / 4, (items + WARPS - 1) / WARPS)));
 
   // Independent host builders, each uploading what it builds: cells and the
   // firm segments; deletion units; target strata; and for the generic
@@ -526,7 +535,7 @@ std::shared_ptr<DeviceEngine> make_device_engine(const Compressed& p, const JlaP
       std::vector<uint32_t> sfirst(fptr.size(), 0);
       for (size_t f = 0; f + 1 < fptr.size(); ++f)
         sfirst[f + 1] = sfirst[f] + (fptr[f + 1] - fptr[f] + SEG - 1) / SEG;
-      build_piece_levels(sfirst, e->firm_pieces, s, h2d);
+      build_hub_rows(sfirst, e->firm_hubs, s, h2d);
     }
     {
       std::vector<double> fd(p.firms, 0.0);
@@ -963,8 +972,7 @@ BlockWork& get_work(DeviceEngine& e) {
   w->tot.alloc(size_t(QMAX + 4) * K);
   w->seg_buf.alloc(size_t(e.lap_seg.count) * K);
   w->fseg_out.alloc(size_t(e.firm_seg.count) * K);
-  w->piece2.alloc(size_t(std::max<uint32_t>(e.firm_pieces.n2, 1)) * K);
-  w->piece3.alloc(size_t(std::max<uint32_t>(e.firm_pieces.n3, 1)) * K);
+  w->hub_sums.alloc(size_t(std::max<uint32_t>(e.firm_hubs.count, 1)) * K);
   w->pack.alloc(pack_size(K));
   double* st = w->st = w->pack.p;
   int* ist = w->ist = reinterpret_cast<int*>(st + 8 * K);
@@ -1447,15 +1455,12 @@ void firm_gather(DeviceEngine& e, BlockWork& w, Launch L, const double* coef, co
   k_seg_firm<K, OP><<<L.grid, THREADS, 0, L.s>>>(e.firm_seg.count, e.firm_seg.begin.p, e.firm_seg.end.p,
                                                   e.firm_cells.p, e.cell_worker.p, coef, src, total, inv_total,
                                                   w.fseg_out.p);
-  const PieceLevels& pl = e.firm_pieces;
-  if (pl.rows) {
-    k_piece_sum<K><<<L.grid, THREADS, 0, L.s>>>(pl.n2, pl.begin2.p, pl.end2.p, w.fseg_out.p, w.piece2.p);
-    k_piece_sum<K><<<L.grid, THREADS, 0, L.s>>>(pl.n3, pl.begin3.p, pl.end3.p, w.piece2.p, w.piece3.p);
-  }
+  const HubRows& hub = e.firm_hubs;
+  if (hub.count)
+    k_hub_rows<K><<<hub.count, HUB_THREADS, 0, L.s>>>(hub.row.p, e.firm_seg.row_first.p, w.fseg_out.p, w.hub_sums.p);
   k_seg_firm_finish<K, MODE><<<L.grid, THREADS, 0, L.s>>>(e.F, e.kept, e.firm_seg.row_first.p, w.fseg_out.p,
-                                                          pl.rows ? pl.slot.p : nullptr, pl.top_first.p,
-                                                          w.piece3.p, bF, bW, e.kept_worker.p, e.firm_diag.p, psi,
-                                                          out, partial);
+                                                          hub.count ? hub.slot.p : nullptr, w.hub_sums.p, bF, bW,
+                                                          e.kept_worker.p, e.firm_diag.p, psi, out, partial);
   CK_LAUNCH();
 }
 
@@ -1507,7 +1512,7 @@ void launch_columns(DeviceEngine& e, BlockWork& w, Launch L, int ncols, double t
 template <int K>
 BlockOutcome solve_block(DeviceEngine& e, BlockWork& w, int ncols, const SolveOptions& o, SolveTimings& tm,
                          const std::function<void(int)>* balance = nullptr) {
-  Launch L{grid_blocks(), e.stream};
+  Launch L{e.grid, e.stream};
   BlockOutcome out;
   // hybrid RHS (Schur reduction of the worker block) and its column sums
   firm_gather<K, 1, 1>(e, w, L, e.cell_scale.p, w.bW.p, nullptr, 0.0, w.bF.p, w.bW.p, nullptr, w.b.p, e.partial.p);
@@ -1774,7 +1779,7 @@ void autotune(DeviceEngine& e, SolveOptions& o, SolveTimings* tm = nullptr) {
       e.tuned = 0;
     } else {
       BlockWork& w = get_work<K>(e);
-      Launch L{grid_blocks(), e.stream};
+      Launch L{e.grid, e.stream};
       const PhiloxKey key = philox_key(o.seed);
       int best = 0;
       SolveTimings scratch;
@@ -1815,7 +1820,7 @@ template <int K>
 void run_leverage(DeviceEngine& e, const SolveOptions& o, SolveResult& res, uint64_t tag_first_probe_unused) {
   (void)tag_first_probe_unused;
   BlockWork& w = get_work<K>(e);
-  Launch L{grid_blocks(), e.stream};
+  Launch L{e.grid, e.stream};
   PhiloxKey key = philox_key(o.seed);
   const uint32_t end = o.probe_end ? o.probe_end : o.probes;
   for (uint32_t first = o.probe_begin; first < end; first += K) {
@@ -1851,7 +1856,7 @@ template <int K>
 void run_target(DeviceEngine& e, const SolveOptions& o, SolveResult& res, double y_center = 0.0) {
   constexpr int H = K / 2;
   BlockWork& w = get_work<K>(e);
-  Launch L{grid_blocks(), e.stream};
+  Launch L{e.grid, e.stream};
   PhiloxKey key = philox_key(o.seed);
   double invT = 1.0 / e.target_total;
   if (res.target_draws.size() != o.probes) res.target_draws.assign(o.probes, Components{});
@@ -2236,7 +2241,7 @@ __global__ void k_scale_copy(size_t n, const double* __restrict__ src, double s,
 template <int K>
 void run_exact(DeviceEngine& e, const Compressed& p, const SolveOptions& o, SolveResult& res) {
   BlockWork& w = get_work<K>(e);
-  Launch L{grid_blocks(), e.stream};
+  Launch L{e.grid, e.stream};
   DBuf<double> cmass(e.C), wshare(e.W), fshare(e.F);
   k_scale_copy<<<L.grid, THREADS, 0, L.s>>>(e.C, e.cell_target.p, 1.0 / p.target_total, cmass.p);
   k_gather<1><<<L.grid, THREADS, 0, L.s>>>(e.W, e.worker_ptr.p, nullptr, cmass.p, wshare.p);
@@ -2312,7 +2317,7 @@ void run_exact(DeviceEngine& e, const Compressed& p, const SolveOptions& o, Solv
 // state's status (2 local, 5 nonsmooth adjustment, 6 nonfinite derivative)
 // and records the shares' extremes in the attachment.
 uint32_t numerical_derivative(DeviceEngine& e, const SolveOptions& o, NumericalAttachment& na) {
-  Launch L{grid_blocks(), e.stream};
+  Launch L{e.grid, e.stream};
   if (!e.num_stats.p) e.num_stats.alloc(8);
   const unsigned long long inf = 0x7ff0000000000000ull;
   unsigned long long init[NUM_STATS] = {0, inf, e.generic ? order_key(INFINITY) : inf, 0, 0}, got[NUM_STATS];
@@ -2355,7 +2360,7 @@ uint32_t numerical_derivative(DeviceEngine& e, const SolveOptions& o, NumericalA
 template <int K>
 bool numerical_replay(DeviceEngine& e, const SolveOptions& o, SolveResult& res, std::vector<Primitive> (&scores)[2]) {
   BlockWork& w = get_work<K>(e);
-  Launch L{grid_blocks(), e.stream};
+  Launch L{e.grid, e.stream};
   PhiloxKey key = philox_key(o.seed);
   NumericalAttachment& na = res.numerical;
   std::vector<double> out(6 * K);
@@ -2419,7 +2424,7 @@ bool numerical_replay_blocks(DeviceEngine& e, const SolveOptions& o, SolveResult
 template <int K>
 void numerical_finish(DeviceEngine& e, const JlaPlan& plan, const SolveOptions& o, double outcome_mean,
                       uint32_t state_status, SolveResult& res) {
-  Launch L{grid_blocks(), e.stream};
+  Launch L{e.grid, e.stream};
   NumericalAttachment& na = res.numerical;
   const uint32_t r = o.probes;
   na.present = true;
@@ -2465,7 +2470,7 @@ void run_jla(DeviceEngine& e, const Compressed& p, const JlaPlan& plan, const So
              SolveResult& res,
              bool detail) {
   SolveOptions o = o_request;  // the autotuner fixes o.precision before the leverage phase
-  Launch L{grid_blocks(), e.stream};
+  Launch L{e.grid, e.stream};
   auto now = [] { return std::chrono::steady_clock::now(); };
   auto t0 = now();
   // ---- full fit (one column); a phase-2 shard reuses the fit of its phase 1
@@ -2616,7 +2621,7 @@ void setup_controls(DeviceEngine& e, const SolveOptions& o, SolveTimings& tm) {
     e.controls_ready = true;
     return;
   }
-  Launch L{grid_blocks(), e.stream};
+  Launch L{e.grid, e.stream};
   BlockWork& w8 = get_work<8>(e);
   const int q = e.q;
   k_cell_controls<<<L.grid, THREADS, 0, L.s>>>(e.C, q, e.cell_rows_ptr.p, e.cell_rows.p, e.row_freq.p, e.Qd.p,
@@ -2684,7 +2689,7 @@ void run_projection(DeviceEngine& e, const Compressed& p, const SolveOptions& o,
     fail(RESOURCE_LIMIT, "generic_jla_projection", "the device projection handles at most 31 covariates");
   if (e.proj_coef.size() != size_t(cols))
     fail(INTERNAL_INVARIANT_FAILED, "generic_jla_projection", "projection coefficient state is incomplete");
-  Launch L{grid_blocks(), e.stream};
+  Launch L{e.grid, e.stream};
   if (e.proj_loaded != &pp) {
     e.proj_wrhs.alloc(pp.worker_rhs.size());
     e.proj_frhs.alloc(pp.firm_rhs.size());
@@ -2790,7 +2795,7 @@ void run_generic(DeviceEngine& e, const Compressed& p, const JlaPlan& plan, cons
              SolveResult& res,
                  bool detail) {
   SolveOptions o = o_request;  // the autotuner fixes o.precision before the leverage phase
-  Launch L{grid_blocks(), e.stream};
+  Launch L{e.grid, e.stream};
   auto now = [] { return std::chrono::steady_clock::now(); };
   auto t0 = now();
   setup_controls(e, o, res.timings);
@@ -3101,7 +3106,7 @@ __global__ void k_fill_pattern(uint32_t n, double* __restrict__ b) {
 template <int K>
 void kernel_benchmark_k(DeviceEngine& e, int kernel, int launches, double* ms, double* bytes) {
   BlockWork& w = get_work<K>(e);
-  Launch L{grid_blocks(), e.stream};
+  Launch L{e.grid, e.stream};
   DBuf<char> flush(size_t(256) << 20);  // larger than the 126 MB L2
   double nnz = double(e.L_col.n), n = double(e.n), nseg = double(e.lap_seg.count);
   PhiloxKey key = philox_key(8675309);

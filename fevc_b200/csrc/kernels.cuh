@@ -274,8 +274,9 @@ __device__ __forceinline__ void redundant_finish(const double* __restrict__ part
   int per = blockDim.x / W;  // >= 1 when blockDim >= W
   const int o = threadIdx.x % W, g = threadIdx.x / W;
   // the loads of U partials are issued before their sum, so a thread waits
-  // for one L2 round trip per U blocks instead of one per block
-  constexpr int U = 8;
+  // for one L2 round trip per U blocks instead of one per block (148 blocks,
+  // 64 columns: one for one value a column, two for two)
+  constexpr int U = 10;
   double acc = 0.0;
   if (g < per)
     for (int b0 = g; b0 < blocks; b0 += U * per) {
