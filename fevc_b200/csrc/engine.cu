@@ -1731,19 +1731,28 @@ inline bool shared_signs(const DeviceEngine& e, uint32_t first) { return e.obser
 
 template <int K>
 void leverage_rhs(DeviceEngine& e, BlockWork& w, Launch L, PhiloxKey key, uint32_t first, int ncols) {
+  // where every cell is one deletion unit the units' atoms are the cells'
+  const bool one_unit = !e.observation && e.G == e.C;
+  const double* cells = one_unit ? w.unit_atoms.p : w.cell_val.p;
   if (shared_signs(e, first)) {
     if (!e.copy_bits.p) e.copy_bits.alloc(e.physical);
     k_obs_leverage_atoms<K><<<L.grid, THREADS, 0, L.s>>>(e.C, e.unit_ptr.p, e.unit_rank.p, e.unit_count.p,
                                                          e.unit_offset.p, e.unit_phys.p, key, first, ncols,
                                                          reinterpret_cast<uint8_t*>(e.copy_bits.p), w.cell_val.p);
   } else {
-    k_leverage_atoms<K><<<L.grid, THREADS, 0, L.s>>>(e.C, e.unit_ptr.p, e.unit_rank.p, e.unit_count.p,
-                                                     e.observation ? e.unit_offset.p : nullptr, key, TAG_LEVERAGE,
-                                                     first, ncols, e.observation ? nullptr : w.unit_atoms.p,
-                                                     w.cell_val.p);
+    auto go = [&](auto kernel) {
+      kernel<<<L.grid, THREADS, 0, L.s>>>(e.C, e.unit_ptr.p, e.unit_rank.p, e.unit_count.p,
+                                          e.observation ? e.unit_offset.p : nullptr, key, TAG_LEVERAGE, first, ncols,
+                                          e.observation ? nullptr : w.unit_atoms.p,
+                                          one_unit ? nullptr : w.cell_val.p);
+    };
+    if (K >= 4 && first % 4 == 0)
+      go(k_leverage_atoms<K, (K >= 4)>);
+    else
+      go(k_leverage_atoms<K, false>);
   }
-  k_gather<K><<<L.grid, THREADS, 0, L.s>>>(e.W, e.worker_ptr.p, nullptr, w.cell_val.p, w.bW.p);
-  firm_gather<K, 0, 0>(e, w, L, nullptr, w.cell_val.p, nullptr, 0.0, nullptr, nullptr, nullptr, w.bF.p, nullptr);
+  k_gather<K><<<L.grid, THREADS, 0, L.s>>>(e.W, e.worker_ptr.p, nullptr, cells, w.bW.p);
+  firm_gather<K, 0, 0>(e, w, L, nullptr, cells, nullptr, 0.0, nullptr, nullptr, nullptr, w.bF.p, nullptr);
 }
 
 // The solver-form autotuner (precision option 2).  On a generation's first
@@ -1874,8 +1883,14 @@ void run_target(DeviceEngine& e, const SolveOptions& o, SolveResult& res, double
   for (uint32_t first = o.probe_begin; first < end; first += H) {
     int np = int(std::min<uint32_t>(H, end - first));
     double* sums = e.draw_sums.p + outcomes.size() * slot;
-    k_target_direction<H><<<L.grid, THREADS, 0, L.s>>>(e.C, e.tgt_ptr.p, e.tgt_rank.p, e.tgt_count.p,
-                                                       e.tgt_scale.p, key, first, np, w.dir.p);
+    auto direction = [&](auto kernel) {
+      kernel<<<L.grid, THREADS, 0, L.s>>>(e.C, e.tgt_ptr.p, e.tgt_rank.p, e.tgt_count.p, e.tgt_scale.p, key, first,
+                                          np, w.dir.p);
+    };
+    if (H >= 4 && first % 4 == 0)
+      direction(k_target_direction<H, (H >= 4)>);
+    else
+      direction(k_target_direction<H, false>);
     // direction totals: sum_c d and the reference scale sum_c |d| + |sum_c d|
     k_colsum_abs<H><<<L.grid, THREADS, 0, L.s>>>(e.C, w.dir.p, e.partial.p);
     finish(e.partial.p, L.grid, 2 * H, w.tot.p, L.s);
@@ -3220,9 +3235,9 @@ void kernel_benchmark_k(DeviceEngine& e, int kernel, int launches, double* ms, d
                                                                reinterpret_cast<uint8_t*>(e.copy_bits.p),
                                                                w.cell_val.p);
         else
-          k_leverage_atoms<K><<<L.grid, THREADS, 0, L.s>>>(e.C, e.unit_ptr.p, e.unit_rank.p, e.unit_count.p,
-                                                           nullptr, key, TAG_LEVERAGE, 0, K, w.unit_atoms.p,
-                                                           w.cell_val.p);
+          k_leverage_atoms<K, true><<<L.grid, THREADS, 0, L.s>>>(e.C, e.unit_ptr.p, e.unit_rank.p, e.unit_count.p,
+                                                                 nullptr, key, TAG_LEVERAGE, 0, K, w.unit_atoms.p,
+                                                                 e.G == e.C ? nullptr : w.cell_val.p);
         break;
       case 4:
         // the moment pass the solver runs (reading the recorded signs)

@@ -249,15 +249,16 @@ __global__ void k_adjust(AdjustParams prm, const uint32_t* __restrict__ unit_ptr
 // Target directions for H probes starting at `first` (reference
 // `target_directions_with_interrupt`, engine.rs:2621-2700): per cell
 // d[c*H + j] = sum over the cell's strata of sqrt(per_copy/T) * atom.
-template <int H>
+// ALIGNED as in k_leverage_atoms.
+template <int H, bool ALIGNED>
 __global__ void k_target_direction(uint32_t cells, const uint32_t* __restrict__ tgt_ptr,
                                    const uint64_t* __restrict__ tgt_rank, const uint64_t* __restrict__ tgt_count,
                                    const double* __restrict__ tgt_scale, PhiloxKey key, uint64_t first, int nprobes,
                                    double* __restrict__ d) {
   // probe first + j sits in lane (first + j) % 4 of Philox block (first + j) / 4;
   // a block of H probes starting off a multiple of four spans one more block
-  constexpr int B = (H + 3) / 4 + 1;
-  const int off = int(first % 4);
+  constexpr uint32_t B = ALIGNED ? H / 4 : (H + 3) / 4 + 1;
+  const int off = ALIGNED ? 0 : int(first % 4);
   size_t total = size_t(cells) * B;
   for (size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += size_t(gridDim.x) * blockDim.x) {
     uint32_t c = uint32_t(t / B);
@@ -270,6 +271,13 @@ __global__ void k_target_direction(uint32_t cells, const uint32_t* __restrict__ 
       double sc = tgt_scale[s];
 #pragma unroll
       for (int l = 0; l < 4; ++l) acc[l].add(sc * double(a[l]));
+    }
+    if constexpr (ALIGNED) {
+      double v[4];
+#pragma unroll
+      for (int l = 0; l < 4; ++l) v[l] = 4 * b + l < nprobes ? acc[l].finish() : 0.0;
+      store4(d + size_t(c) * H + 4 * b, v);
+      continue;
     }
 #pragma unroll
     for (int l = 0; l < 4; ++l) {

@@ -16,6 +16,7 @@
 #include "counter_rng.h"
 #include "device.cuh"
 #include "generic.cuh"
+#include "kernels.cuh"
 
 namespace fevcb {
 
@@ -49,9 +50,30 @@ __global__ void k_obs_leverage_atoms(uint32_t cells, const uint32_t* __restrict_
   for (size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += size_t(gridDim.x) * blockDim.x) {
     const uint32_t c = uint32_t(t / Q);
     const int q = int(t % Q);
-    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    // the cell's sums as integers (exact), one conversion a column at the end
+    int64_t acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (uint32_t g = unit_ptr[c]; g < unit_ptr[c + 1]; ++g) {
       const uint64_t ent = unit_rank[g], off = unit_offset[g], n = unit_count[g], ph = unit_phys[g];
+      if (n == 1) {
+        // one copy (a row without frequency weights): its eight bits are the
+        // byte, and the atoms are 2 bit - 1; 32-bit shifts on the word's half
+        uint64_t b0[4], b1[4] = {0, 0, 0, 0};
+        philox_block(key, ent, pblock0 + 2 * q, off >> 6, TAG_LEVERAGE, b0);
+        if (K > 4) philox_block(key, ent, pblock0 + 2 * q + 1, off >> 6, TAG_LEVERAGE, b1);
+        const bool high = (off & 32) != 0;
+        const int bit = int(off & 31);
+        uint32_t v = 0;
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+          const uint32_t x = (uint32_t(high ? b0[l] >> 32 : b0[l]) >> bit) & 1u;
+          const uint32_t y = (uint32_t(high ? b1[l] >> 32 : b1[l]) >> bit) & 1u;
+          v |= x << l | y << (4 + l);
+          acc[l] += int32_t(2 * x) - 1;
+          acc[4 + l] += int32_t(2 * y) - 1;
+        }
+        copy_bits[ph * 8 + q] = uint8_t(v);
+        continue;
+      }
       int64_t pos[8] = {0, 0, 0, 0, 0, 0, 0, 0};
       uint64_t cp = off;
       const uint64_t end = off + n;
@@ -78,12 +100,20 @@ __global__ void k_obs_leverage_atoms(uint32_t cells, const uint32_t* __restrict_
         cp = (word << 6) + hi;
       }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] += double(2 * pos[j] - int64_t(n));
+      for (int j = 0; j < 8; ++j) acc[j] += 2 * pos[j] - int64_t(n);
     }
+    if constexpr (K >= 8) {
+      double v[2][4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int col = 8 * q + j;
-      if (col < K) cell_atoms[size_t(c) * K + col] = col < ncols ? acc[j] : 0.0;
+      for (int j = 0; j < 8; ++j) v[j / 4][j % 4] = 8 * q + j < ncols ? double(acc[j]) : 0.0;
+      store4(cell_atoms + size_t(c) * K + 8 * q, v[0]);
+      store4(cell_atoms + size_t(c) * K + 8 * q + 4, v[1]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int col = 8 * q + j;
+        if (col < K) cell_atoms[size_t(c) * K + col] = col < ncols ? double(acc[j]) : 0.0;
+      }
     }
   }
 }
