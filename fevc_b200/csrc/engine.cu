@@ -1873,7 +1873,8 @@ void run_target(DeviceEngine& e, const SolveOptions& o, SolveResult& res, double
   // every block's contraction sums stay on the device until the last block:
   // (u^2, v^2, u v) of the compressed engine, the two sides and their total of
   // the match units with controls, or the fused leave-observation-out sums
-  const size_t slot = e.observation ? size_t(2) * (QMAX + 1) * K : e.generic ? size_t(2) * K : size_t(3) * K;
+  const int Q = e.qa == 0 ? 0 : e.qa <= 4 ? 4 : QMAX;  // controls the fused pass's sums hold
+  const size_t slot = e.observation ? size_t(2) * (Q + 1) * K : e.generic ? size_t(2) * K : size_t(3) * K;
   const size_t blocks = o.probe_begin < end ? (end - o.probe_begin + H - 1) / H : 0;
   if (e.draw_sums.n < slot * blocks) e.draw_sums.alloc(slot * blocks);
   std::vector<BlockOutcome> outcomes;
@@ -1926,11 +1927,19 @@ void run_target(DeviceEngine& e, const SolveOptions& o, SolveResult& res, double
     } else if (e.observation) {
       // one pass over the cells: the control sums and the draws' beta-free parts
       if (!e.partial2.p) e.partial2.alloc(size_t(L.grid) * (QMAX + 1) * 128 + 1024);
-      k_obs_target_cells<K><<<L.grid, THREADS, 0, L.s>>>(e.C, e.qa, e.cell_worker.p, e.cell_firm.p,
-                                                         e.qa > 0 ? e.cellQ.p : nullptr, e.obs_cell_sums.p,
-                                                         w.alpha.p, w.x.p, e.partial.p, e.partial2.p);
-      finish(e.partial.p, L.grid, (QMAX + 1) * K, sums, L.s);
-      finish(e.partial2.p, L.grid, (QMAX + 1) * K, sums + (QMAX + 1) * K, L.s);
+      auto target = [&](auto kernel) {
+        kernel<<<L.grid, THREADS, 0, L.s>>>(e.C, e.qa, warp_chunk(e.C, L.grid), e.cell_worker.p, e.cell_firm.p,
+                                            e.qa > 0 ? e.cellQ.p : nullptr, e.obs_cell_sums.p, w.alpha.p, w.x.p,
+                                            e.partial.p, e.partial2.p);
+      };
+      if (Q == 0)
+        target(k_obs_target_cells<K, 0>);
+      else if (Q == 4)
+        target(k_obs_target_cells<K, 4>);
+      else
+        target(k_obs_target_cells<K, QMAX>);
+      finish(e.partial.p, L.grid, (Q + 1) * K, sums, L.s);
+      finish(e.partial2.p, L.grid, (Q + 1) * K, sums + (Q + 1) * K, L.s);
       if (o.numerical) {  // the attachment's per-row target folds of this block
         k_solve_beta<K><<<1, 512, 0, L.s>>>(e.qa, sinv, sums, e.beta_buf.p);
         k_obs_num_folds<K><<<L.grid, THREADS, 0, L.s>>>(e.C, e.qa, uint64_t(first), np, e.unit_ptr.p,
@@ -1976,9 +1985,9 @@ void run_target(DeviceEngine& e, const SolveOptions& o, SolveResult& res, double
     } else {
       std::copy_n(f, std::min<size_t>(slot, 2 * K), g2.begin());
       if (e.observation) {
-        const double* A = f + QMAX * K;
-        const double* B = f + (QMAX + 1) * K;
-        const double* Atot = f + (2 * QMAX + 1) * K;
+        const double* A = f + Q * K;
+        const double* B = f + (Q + 1) * K;
+        const double* Atot = f + (2 * Q + 1) * K;
         for (int k = 0; k < e.qa; ++k)
           for (int j = 0; j < K; ++j) {
             double v = 0.0;

@@ -548,60 +548,97 @@ __global__ void k_obs_cell_target_sums(uint32_t cells, int q, const uint32_t* __
 // u_worker + u_firm.  With beta = -S^{-1} t the host forms the draws
 // A + 2 B'beta + beta' S2 beta (the cell sum of S0 u^2 + 2 u S1'beta plus the
 // cell-independent quadratic term).
-// partial: [blk][9][K] = (t_0 .. t_7, A); partial2: [blk][9][K] = (B_0 .. B_7, A_tot).
-template <int K>
-__global__ void k_obs_target_cells(uint32_t cells, int q, const uint32_t* __restrict__ cell_worker,
-                                   const uint32_t* __restrict__ cell_firm, const double* __restrict__ CQ,
-                                   const double* __restrict__ sums, const double* __restrict__ alpha,
-                                   const double* __restrict__ psi, double* __restrict__ partial,
-                                   double* __restrict__ partial2) {
+// partial: [blk][Q + 1][K] = (t_0 .., A); partial2: [blk][Q + 1][K] = (B_0 ..,
+// A_tot), Q >= q the controls the accumulators hold (0, 4 or 8): at eight, 72
+// registers of sums left two blocks an SM and the pass waited for its rows
+// (1,330 us for 2.8M cells and four controls; 610 us so).  With one warp a
+// cell, the cells' workers and firms are loaded `chunk` at a time lane-parallel
+// and two cells' rows are in flight.
+template <int K, int Q>
+__global__ void __launch_bounds__(THREADS) k_obs_target_cells(
+    uint32_t cells, int q, uint32_t chunk, const uint32_t* __restrict__ cell_worker,
+    const uint32_t* __restrict__ cell_firm, const double* __restrict__ CQ, const double* __restrict__ sums,
+    const double* __restrict__ alpha, const double* __restrict__ psi, double* __restrict__ partial,
+    double* __restrict__ partial2) {
   constexpr int CPT = Cols<K>::CPT, TPR = Cols<K>::TPR;
   static_assert(CPT <= 2, "pairs of columns must sit in one thread or in adjacent lanes");
-  static_assert(QMAX == 8, "nine sums per reduction");
-  double v1[QMAX + 1][CPT], v2[QMAX + 1][CPT];
+  double v1[Q + 1][CPT], v2[Q + 1][CPT];
 #pragma unroll
-  for (int k = 0; k <= QMAX; ++k)
+  for (int k = 0; k <= Q; ++k)
 #pragma unroll
     for (int c = 0; c < CPT; ++c) v1[k][c] = v2[k][c] = 0.0;
   const int c0 = int(threadIdx.x % TPR) * CPT;
-  size_t total = size_t(cells) * TPR, stride = size_t(gridDim.x) * blockDim.x;
-  for (size_t base = size_t(blockIdx.x) * blockDim.x; base < total; base += stride) {
-    size_t t = base + threadIdx.x;
-    bool live = t < total;
-    size_t c = live ? t / TPR : 0;
-    double u[CPT], s0 = 0.0;
+  // u: the cell's prediction at this thread's columns; sc: its sums
+  auto add = [&](size_t c, const double (&u)[CPT]) {
+    const double* sc = sums + c * size_t(1 + q);
+    const double s0 = sc[0];
 #pragma unroll
-    for (int cc = 0; cc < CPT; ++cc) u[cc] = 0.0;
-    if (live) {
-      const double* sc = sums + c * size_t(1 + q);
-      s0 = sc[0];
-      size_t wb = size_t(cell_worker[c]) * K + c0, fb = size_t(cell_firm[c]) * K + c0;
+    for (int k = 0; k < Q; ++k)
+      if (k < q) {
+        const double cq = CQ[c * QMAX + k], s1 = sc[1 + k];
 #pragma unroll
-      for (int cc = 0; cc < CPT; ++cc) u[cc] = alpha[wb + cc] + psi[fb + cc];
+        for (int cc = 0; cc < CPT; ++cc) {
+          v1[k][cc] += u[cc] * cq;
+          v2[k][cc] += u[cc] * s1;
+        }
+      }
 #pragma unroll
-      for (int k = 0; k < QMAX; ++k)
-        if (k < q) {
-          const double cq = CQ[c * QMAX + k], s1 = sc[1 + k];
+    for (int cc = 0; cc < CPT; ++cc) v1[Q][cc] += s0 * u[cc] * u[cc];
+    return s0;
+  };
+  if constexpr (TPR == 32) {
+    const int lane = threadIdx.x & 31;
+    const size_t nwarps = size_t(gridDim.x) * blockDim.x / 32;
+    for (size_t i0 = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32 * chunk; i0 < cells; i0 += nwarps * chunk) {
+      const int cnt = int(cells - i0 < chunk ? cells - i0 : chunk);
+      uint32_t my_w = 0, my_f = 0;
+      if (lane < cnt) {
+        my_w = cell_worker[i0 + lane];
+        my_f = cell_firm[i0 + lane];
+      }
+      constexpr int U = 2;
+      for (int i = 0; i < cnt; i += U) {
+        double av[U][CPT], pv[U][CPT];
 #pragma unroll
-          for (int cc = 0; cc < CPT; ++cc) {
-            v1[k][cc] += u[cc] * cq;
-            v2[k][cc] += u[cc] * s1;
-          }
+        for (int x = 0; x < U; ++x) {
+          const int src = i + x < cnt ? i + x : i;  // the last odd cell is read twice, added once
+          load_cols<K, double>(alpha, __shfl_sync(0xffffffffu, my_w, src), c0, av[x]);
+          load_cols<K, double>(psi, __shfl_sync(0xffffffffu, my_f, src), c0, pv[x]);
         }
 #pragma unroll
-      for (int cc = 0; cc < CPT; ++cc) v1[QMAX][cc] += s0 * u[cc] * u[cc];
+        for (int x = 0; x < U; ++x)
+          if (i + x < cnt) {
+            double u[CPT];
+#pragma unroll
+            for (int cc = 0; cc < CPT; ++cc) u[cc] = av[x][cc] + pv[x][cc];
+            const double s0 = add(i0 + i + x, u);
+            const double uu = CPT == 2 ? u[0] + u[CPT - 1] : u[0] + __shfl_xor_sync(0xffffffffu, u[0], 1);
+            if (CPT == 2 || (c0 & 1) == 0) v2[Q][0] += s0 * uu * uu;
+          }
+      }
     }
-    if (CPT == 2) {
-      const double uu = u[0] + u[CPT - 1];
-      v2[QMAX][0] += s0 * uu * uu;
-    } else {
+  } else {
+    size_t total = size_t(cells) * TPR, stride = size_t(gridDim.x) * blockDim.x;
+    for (size_t base = size_t(blockIdx.x) * blockDim.x; base < total; base += stride) {
+      size_t t = base + threadIdx.x;
+      bool live = t < total;
+      size_t c = live ? t / TPR : 0;
+      double u[CPT], s0 = 0.0;
+#pragma unroll
+      for (int cc = 0; cc < CPT; ++cc) u[cc] = 0.0;
+      if (live) {
+        size_t wb = size_t(cell_worker[c]) * K + c0, fb = size_t(cell_firm[c]) * K + c0;
+#pragma unroll
+        for (int cc = 0; cc < CPT; ++cc) u[cc] = alpha[wb + cc] + psi[fb + cc];
+        s0 = add(c, u);
+      }
       const double uo = __shfl_xor_sync(0xffffffffu, u[0], 1);
       const double uu = u[0] + uo;
-      if ((c0 & 1) == 0) v2[QMAX][0] += s0 * uu * uu;
+      if ((c0 & 1) == 0) v2[Q][0] += s0 * uu * uu;
     }
   }
-  block_reduce_cols<K, QMAX + 1>(v1, partial);
-  block_reduce_cols<K, QMAX + 1>(v2, partial2);
+  block_reduce_cols<K, Q + 1>(v1, partial);
+  block_reduce_cols<K, Q + 1>(v2, partial2);
 }
 
 // Cell-level control sums of the target solutions: partial[blk][k][col] =
