@@ -243,6 +243,22 @@ __global__ void __launch_bounds__(THREADS) k_spmm_rows_dot(uint32_t n, const uin
   block_reduce_cols<K, 1>(v, partial);
 }
 
+// Columns c0 .. c0 + CPT - 1 of vertex j, as one vector store where the width
+// allows (two scalar stores of a lane's pair touch every sector twice).
+template <int K, typename V>
+__device__ __forceinline__ void put_cols(V* y, size_t j, int c0, const double (&v)[Cols<K>::CPT]) {
+  constexpr int CPT = Cols<K>::CPT;
+  V* dst = y + j * K + c0;
+  if constexpr (CPT == 2 && sizeof(V) == 8) {
+    *reinterpret_cast<double2*>(dst) = make_double2(v[0], v[1]);
+  } else if constexpr (CPT == 2 && sizeof(V) == 4) {
+    *reinterpret_cast<float2*>(dst) = make_float2(float(v[0]), float(v[1]));
+  } else {
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) dst[c] = V(v[c]);
+  }
+}
+
 // V is the storage type of the Laplacian values and of the iteration vectors
 // x, r, p and the segment products: double for the FP64 solve, float for the
 // inner solve of mixed-precision refinement.  Products, dots and step
@@ -407,11 +423,9 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_pcg_persistent(Persisten
         warp_gather<K, V>(my_j, my_a, e1 - b1, a.p, c0, acc);
         double pr[CPT];
         load_cols<K, V>(a.p, row, c0, pr);
+        put_cols<K, V>(a.seg_buf, id1, c0, acc);
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) {
-          a.seg_buf[size_t(id1) * K + c0 + c] = V(acc[c]);
-          v[0][c] += pr[c] * (d * pr[c] - acc[c]);
-        }
+        for (int c = 0; c < CPT; ++c) v[0][c] += pr[c] * (d * pr[c] - acc[c]);
         f1 = f2;
         b1 = b2;
         e1 = e2;
@@ -534,23 +548,28 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_pcg_persistent(Persisten
       const size_t row = balanced ? a.light_rows[li] : li;
       uint32_t s0 = a.row_first[row], s1 = a.row_first[row + 1];
       double dr = double(a.diag[row]), di = double(a.dinv[row]);
-      size_t o = row * K + c0;
-      double q[CPT];
+      double q[CPT], pv[CPT], xv[CPT], rv[CPT];
+      load_cols<K, V>(a.p, uint32_t(row), c0, pv);
+      load_cols<K, V>(a.x, uint32_t(row), c0, xv);
+      load_cols<K, V>(a.r, uint32_t(row), c0, rv);
 #pragma unroll
-      for (int c = 0; c < CPT; ++c) q[c] = dr * double(a.p[o + c]);
-      for (uint32_t sg = s0; sg < s1; ++sg)
+      for (int c = 0; c < CPT; ++c) q[c] = dr * pv[c];
+      for (uint32_t sg = s0; sg < s1; ++sg) {
+        double sv[CPT];
+        load_cols<K, V>(a.seg_buf, sg, c0, sv);
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) q[c] -= double(a.seg_buf[size_t(sg) * K + c0 + c]);
+        for (int c = 0; c < CPT; ++c) q[c] -= sv[c];
+      }
 #pragma unroll
       for (int c = 0; c < CPT; ++c) {
-        double al = s_alpha[c0 + c];
-        a.x[o + c] = V(double(a.x[o + c]) + al * double(a.p[o + c]));
-        V rv = V(double(a.r[o + c]) - al * q[c]);
-        a.r[o + c] = rv;
-        double ri = double(rv);
-        w[0][c] += ri * (di * ri);
-        w[1][c] += ri * ri;
+        const double al = s_alpha[c0 + c];
+        xv[c] += al * pv[c];
+        rv[c] = double(V(rv[c] - al * q[c]));
+        w[0][c] += rv[c] * (di * rv[c]);
+        w[1][c] += rv[c] * rv[c];
       }
+      put_cols<K, V>(a.x, row, c0, xv);
+      put_cols<K, V>(a.r, row, c0, rv);
     }
     block_reduce_cols_big<K, 2>(w, a.partial_b, (double(*)[2][K])s_red);
     grid.sync();
@@ -581,11 +600,13 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_pcg_persistent(Persisten
     }
     // ---- C: p = dinv r + beta p
     for (size_t row = gid; row < a.n; row += ngroups) {
-      double di = double(a.dinv[row]);
-      size_t o = row * K + c0;
+      const double di = double(a.dinv[row]);
+      double pv[CPT], rv[CPT];
+      load_cols<K, V>(a.r, uint32_t(row), c0, rv);
+      load_cols<K, V>(a.p, uint32_t(row), c0, pv);
 #pragma unroll
-      for (int c = 0; c < CPT; ++c)
-        a.p[o + c] = V(di * double(a.r[o + c]) + s_beta[c0 + c] * double(a.p[o + c]));
+      for (int c = 0; c < CPT; ++c) pv[c] = di * rv[c] + s_beta[c0 + c] * pv[c];
+      put_cols<K, V>(a.p, row, c0, pv);
     }
     grid.sync();
   }
