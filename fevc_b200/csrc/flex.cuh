@@ -229,21 +229,33 @@ __device__ __forceinline__ void row_pass(const Arg& a, Sh<K>& sh, const VO* seg,
     }
     __syncthreads();
   }
-  const size_t warp = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const size_t nw = (size_t(gridDim.x) * blockDim.x) >> 5;
-  for (size_t li = warp; li < a.nlight; li += nw) {
-    const uint32_t row = a.light_rows[li];
-    const uint32_t s0 = a.row_first[row], s1 = a.row_first[row + 1];
-    double sum[CPT];
-#pragma unroll
-    for (int c = 0; c < CPT; ++c) sum[c] = 0.0;
-    for (uint32_t sg = s0; sg < s1; ++sg) {
-      double sv[CPT];
-      load_cols<K, VO>(seg, sg, c0, sv);
-#pragma unroll
-      for (int c = 0; c < CPT; ++c) sum[c] += sv[c];
+  // 32 rows' index and segment range loaded lane-parallel and broadcast: a row
+  // waits for its vectors alone, not for its index, its range and then them
+  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t base = warp; base < a.nlight; base += nw * 32) {
+    const uint32_t mine = base + uint32_t(lane) * nw;
+    uint32_t my_row = 0, my_s0 = 0, my_s1 = 0;
+    if (mine < a.nlight) {
+      my_row = __ldg(a.light_rows + mine);
+      my_s0 = __ldg(a.row_first + my_row);
+      my_s1 = __ldg(a.row_first + my_row + 1);
     }
-    f(row, sum);
+    const int cnt = int(min((a.nlight - base + nw - 1) / nw, 32u));
+    for (int i = 0; i < cnt; ++i) {
+      const uint32_t row = __shfl_sync(0xffffffffu, my_row, i);
+      const uint32_t s0 = __shfl_sync(0xffffffffu, my_s0, i), s1 = __shfl_sync(0xffffffffu, my_s1, i);
+      double sum[CPT];
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) sum[c] = 0.0;
+      for (uint32_t sg = s0; sg < s1; ++sg) {
+        double sv[CPT];
+        load_cols<K, VO>(seg, sg, c0, sv);
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) sum[c] += sv[c];
+      }
+      f(row, sum);
+    }
   }
 }
 

@@ -543,15 +543,12 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_pcg_persistent(Persisten
         __syncthreads();
       }
     }
-    const size_t nrows = balanced ? a.nlight : a.n;
-    for (size_t li = gid; li < nrows; li += ngroups) {
-      const size_t row = balanced ? a.light_rows[li] : li;
-      uint32_t s0 = a.row_first[row], s1 = a.row_first[row + 1];
+    auto update = [&](uint32_t row, uint32_t s0, uint32_t s1) {
       double dr = double(a.diag[row]), di = double(a.dinv[row]);
       double q[CPT], pv[CPT], xv[CPT], rv[CPT];
-      load_cols<K, V>(a.p, uint32_t(row), c0, pv);
-      load_cols<K, V>(a.x, uint32_t(row), c0, xv);
-      load_cols<K, V>(a.r, uint32_t(row), c0, rv);
+      load_cols<K, V>(a.p, row, c0, pv);
+      load_cols<K, V>(a.x, row, c0, xv);
+      load_cols<K, V>(a.r, row, c0, rv);
 #pragma unroll
       for (int c = 0; c < CPT; ++c) q[c] = dr * pv[c];
       for (uint32_t sg = s0; sg < s1; ++sg) {
@@ -570,6 +567,25 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_pcg_persistent(Persisten
       }
       put_cols<K, V>(a.x, row, c0, xv);
       put_cols<K, V>(a.r, row, c0, rv);
+    };
+    if (balanced) {
+      // 32 light rows' index and segment range loaded lane-parallel
+      const uint32_t ng = uint32_t(ngroups), lane = threadIdx.x & 31;
+      for (uint32_t base = uint32_t(gid); base < a.nlight; base += ng * 32) {
+        const uint32_t mine = base + lane * ng;
+        uint32_t my_row = 0, my_s0 = 0, my_s1 = 0;
+        if (mine < a.nlight) {
+          my_row = __ldg(a.light_rows + mine);
+          my_s0 = __ldg(a.row_first + my_row);
+          my_s1 = __ldg(a.row_first + my_row + 1);
+        }
+        const int cnt = int(min((a.nlight - base + ng - 1) / ng, 32u));
+        for (int i = 0; i < cnt; ++i)
+          update(__shfl_sync(0xffffffffu, my_row, i), __shfl_sync(0xffffffffu, my_s0, i),
+                 __shfl_sync(0xffffffffu, my_s1, i));
+      }
+    } else {
+      for (size_t row = gid; row < a.n; row += ngroups) update(uint32_t(row), a.row_first[row], a.row_first[row + 1]);
     }
     block_reduce_cols_big<K, 2>(w, a.partial_b, (double(*)[2][K])s_red);
     grid.sync();
