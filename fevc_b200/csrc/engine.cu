@@ -1843,7 +1843,7 @@ void run_leverage(DeviceEngine& e, const SolveOptions& o, SolveResult& res, uint
     }
     e.tuned_block_width = 0;
     if (e.observation && shared_signs(e, first))
-      k_obs_moments_cells<K><<<L.grid, THREADS, 0, L.s>>>(e.C, ncols, e.unit_ptr.p, e.cell_rows.p, e.cell_worker.p,
+      k_obs_moments_cells<K><<<L.grid, THREADS, 0, L.s>>>(e.C, ncols, warp_chunk(e.C, L.grid), e.unit_ptr.p, e.cell_rows.p, e.cell_worker.p,
                                                           e.cell_firm.p, e.unit_phys.p, e.unit_count.p,
                                                           e.copy_bits.p, w.alpha.p, w.x.p, e.obs_row_acc.p,
                                                           e.obs_copy_acc.p);
@@ -3251,7 +3251,7 @@ void kernel_benchmark_k(DeviceEngine& e, int kernel, int launches, double* ms, d
       case 4:
         // the moment pass the solver runs (reading the recorded signs)
         if (e.observation)
-          k_obs_moments_cells<K><<<L.grid, THREADS, 0, L.s>>>(e.C, K, e.unit_ptr.p, e.cell_rows.p, e.cell_worker.p,
+          k_obs_moments_cells<K><<<L.grid, THREADS, 0, L.s>>>(e.C, K, warp_chunk(e.C, L.grid), e.unit_ptr.p, e.cell_rows.p, e.cell_worker.p,
                                                               e.cell_firm.p, e.unit_phys.p, e.unit_count.p,
                                                               e.copy_bits.p, w.alpha.p, w.x.p, e.obs_row_acc.p,
                                                               e.obs_copy_acc.p);

@@ -235,111 +235,159 @@ __global__ void k_obs_moments(uint32_t rows, int ncols, const uint32_t* __restri
   }
 }
 
+// The warp's sums of four values a lane; lane l gets the sum of value l / 8.
+// Values are exchanged while they are halved (six shuffles, where a tree for
+// each value takes twenty).
+__device__ __forceinline__ double warp_sum4(const double (&v)[4]) {
+  const int lane = threadIdx.x & 31;
+  const bool h = lane & 16, q = lane & 8;
+  double a = h ? v[2] : v[0], b = h ? v[3] : v[1];
+  a += __shfl_xor_sync(0xffffffffu, h ? v[0] : v[2], 16);
+  b += __shfl_xor_sync(0xffffffffu, h ? v[1] : v[3], 16);
+  double s = q ? b : a;
+  s += __shfl_xor_sync(0xffffffffu, q ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
 // The same moments over cells, with the block's signs read from copy_bits
-// (k_obs_leverage_atoms wrote them): one warp per cell.  The rows of a cell
-// share its prediction P = alpha_w + psi_f, so P is loaded once per cell, every
+// (k_obs_leverage_atoms wrote them): a warp takes `chunk` (at most 32) cells.
+// The rows of a cell share its prediction P = alpha_w + psi_f, so P is loaded
+// once per cell (the next cell's rows while the current one is summed), every
 // row of the cell gets the same (sum P^2, sum P^4), and each copy's (sum a P,
 // sum a P^3) comes from its sign word (bit j: column j drew +1).  Lane l holds
-// columns l*CPT ..; the warp's sums are fixed xor trees, so the result is
+// columns l*CPT ..; the order of every sum is fixed, so the result is
 // deterministic.  Units are the cell's rows in cell order (unit_ptr), with
 // cell_rows[u] the row of unit u, unit_phys[u] its first copy and
 // unit_count[u] its copies.
+// A unit's four sums (its row's two, its first copy's two) are reduced
+// together, and eight units' (or sixteen further copies') accumulators are
+// loaded before the sums are formed and updated with one 16-byte access a
+// lane.  Bound by the accumulators' and worker rows' memory traffic and the
+// shuffles.
 template <int K>
 __global__ void __launch_bounds__(THREADS) k_obs_moments_cells(
-    uint32_t cells, int ncols, const uint32_t* __restrict__ unit_ptr, const uint32_t* __restrict__ cell_rows,
-    const uint32_t* __restrict__ cell_worker, const uint32_t* __restrict__ cell_firm,
-    const uint64_t* __restrict__ unit_phys, const uint64_t* __restrict__ unit_count,
-    const uint64_t* __restrict__ copy_bits, const double* __restrict__ alpha, const double* __restrict__ psi,
-    double* __restrict__ row_acc, double* __restrict__ copy_acc) {
+    uint32_t cells, int ncols, uint32_t chunk, const uint32_t* __restrict__ unit_ptr,
+    const uint32_t* __restrict__ cell_rows, const uint32_t* __restrict__ cell_worker,
+    const uint32_t* __restrict__ cell_firm, const uint64_t* __restrict__ unit_phys,
+    const uint64_t* __restrict__ unit_count, const uint64_t* __restrict__ copy_bits,
+    const double* __restrict__ alpha, const double* __restrict__ psi, double* __restrict__ row_acc,
+    double* __restrict__ copy_acc) {
   constexpr int CPT = Cols<K>::CPT;
   constexpr int LANES = K / CPT;  // lanes that hold columns
   static_assert(LANES <= 32, "one warp per cell");
+  constexpr uint32_t FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int c0 = lane * CPT;
+  const int slot = lane & 7, kind = lane >> 3;  // lane's accumulator: unit `slot` of eight, sum `kind` of four
   const size_t warp = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const size_t nw = (size_t(gridDim.x) * blockDim.x) >> 5;
-  for (size_t c = warp; c < cells; c += nw) {
-    const uint32_t u0 = unit_ptr[c], u1 = unit_ptr[c + 1];
-    const uint32_t cnt = u1 - u0;
-    // the cell's units, lane-parallel: first copy, copies and its sign word
-    uint64_t my_ph = 0, my_n = 0, my_bits = 0;
-    uint32_t my_row = 0;
-    if (uint32_t(lane) < cnt) {
-      my_ph = unit_phys[u0 + lane];
-      my_n = unit_count[u0 + lane];
-      my_row = cell_rows[u0 + lane];
-      my_bits = my_n ? copy_bits[my_ph] : 0;
+  auto update = [](double* at, double2 a, double v) {
+    if (!at) return;
+    neumaier_add(a.x, a.y, v);
+    *reinterpret_cast<double2*>(at) = a;
+  };
+  for (size_t cb = warp * chunk; cb < cells; cb += nw * chunk) {
+    const int nc = int(cells - cb < chunk ? cells - cb : chunk);
+    uint32_t my_end = 0, my_w = 0, my_f = 0;
+    if (lane < nc) {
+      my_end = unit_ptr[cb + lane + 1];
+      my_w = cell_worker[cb + lane];
+      my_f = cell_firm[cb + lane];
     }
-    const size_t wi = size_t(cell_worker[c]) * K, fi = size_t(cell_firm[c]) * K;
-    double P[CPT], s2 = 0.0, s4 = 0.0;
-#pragma unroll
-    for (int q = 0; q < CPT; ++q) {
-      const int col = c0 + q;
-      P[q] = (lane < LANES && col < ncols) ? alpha[wi + col] + psi[fi + col] : 0.0;
-      const double p2 = P[q] * P[q];
-      s2 += p2;
-      s4 += p2 * p2;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-      s4 += __shfl_xor_sync(0xffffffffu, s4, o);
-    }
-    // row sums: every row of the cell, one lane each
-    for (uint32_t u = u0 + uint32_t(lane); u < u1; u += 32) {
-      const uint32_t r = uint32_t(u - u0) < 32 ? my_row : cell_rows[u];
-      double* a = row_acc + size_t(r) * 4;
-      neumaier_add(a[0], a[1], s2);
-      neumaier_add(a[2], a[3], s4);
-    }
-    // copies, unit after unit (the whole warp on each copy's columns); the
-    // k-th copy's sums stay with lane k, and up to 32 copies' accumulators
-    // are updated together, one lane each
-    uint32_t held = 0;
-    uint64_t my_copy = 0;
-    double my_f1 = 0.0, my_f3 = 0.0;
-    auto flush = [&] {
-      if (uint32_t(lane) < held) {
-        double* a = copy_acc + size_t(my_copy) * 4;
-        neumaier_add(a[0], a[1], my_f1);
-        neumaier_add(a[2], a[3], my_f3);
+    const uint32_t ub = unit_ptr[cb], ue = __shfl_sync(FULL, my_end, nc - 1);
+    double na[CPT], np[CPT];  // the next cell's rows
+    auto fetch = [&](int j) {
+      const uint32_t w = __shfl_sync(FULL, my_w, j & 31), f = __shfl_sync(FULL, my_f, j & 31);
+      if (j < nc && lane < LANES) {
+        load_cols<K, double>(alpha, w, c0, na);
+        load_cols<K, double>(psi, f, c0, np);
       }
-      held = 0;
     };
-    for (uint32_t u = 0; u < cnt; ++u) {
-      uint64_t ph, n, bits;
-      if (u < 32) {
-        ph = __shfl_sync(0xffffffffu, my_ph, int(u));
-        n = __shfl_sync(0xffffffffu, my_n, int(u));
-        bits = __shfl_sync(0xffffffffu, my_bits, int(u));
-      } else {
-        ph = unit_phys[u0 + u];
-        n = unit_count[u0 + u];
-        bits = n ? copy_bits[ph] : 0;
+#pragma unroll
+    for (int q = 0; q < CPT; ++q) na[q] = np[q] = 0.0;
+    fetch(0);
+    int cell = -1;
+    uint32_t cend = ub;  // first unit past the current cell
+    double P[CPT], P3[CPT], s2 = 0.0, s4 = 0.0;
+#pragma unroll
+    for (int q = 0; q < CPT; ++q) P[q] = P3[q] = 0.0;
+    auto signed_sums = [&](uint64_t bits, double& f1, double& f3) {
+      f1 = f3 = 0.0;
+#pragma unroll
+      for (int q = 0; q < CPT; ++q) {
+        const bool plus = (bits >> (c0 + q)) & 1;
+        f1 += plus ? P[q] : -P[q];
+        f3 += plus ? P3[q] : -P3[q];
       }
-      for (uint64_t i = 0; i < n; ++i) {
-        const uint64_t m = (i == 0 ? bits : copy_bits[ph + i]) >> c0;
-        double f1 = 0.0, f3 = 0.0;
+    };
+    for (uint32_t u = ub; u < ue; u += 32) {
+      const int m = int(ue - u < 32 ? ue - u : 32);
+      // the next 32 units, lane-parallel: row, first copy, copies, its sign word
+      uint64_t my_ph = 0, my_n = 0, my_bits = 0;
+      uint32_t my_row = 0;
+      if (lane < m) {
+        my_ph = unit_phys[u + lane];
+        my_n = unit_count[u + lane];
+        my_row = cell_rows[u + lane];
+        my_bits = my_n ? copy_bits[my_ph] : 0;
+      }
+      const uint32_t many = __ballot_sync(FULL, my_n > 1);
+      for (int g = 0; g < m; g += 8) {
+        const uint64_t ph8 = __shfl_sync(FULL, my_ph, g + slot), n8 = __shfl_sync(FULL, my_n, g + slot);
+        const uint32_t row8 = __shfl_sync(FULL, my_row, g + slot);
+        double* at = nullptr;
+        if (g + slot < m) {
+          if (kind < 2)
+            at = row_acc + size_t(row8) * 4 + 2 * kind;
+          else if (n8)
+            at = copy_acc + size_t(ph8) * 4 + 2 * (kind - 2);
+        }
+        const double2 old = at ? *reinterpret_cast<const double2*>(at) : make_double2(0.0, 0.0);
+        double mine = 0.0;
+        const int r1 = m - g < 8 ? m - g : 8;
+        for (int r = 0; r < r1; ++r) {
+          while (u + uint32_t(g + r) >= cend) {
+            cend = __shfl_sync(FULL, my_end, ++cell);
+            s2 = s4 = 0.0;
 #pragma unroll
-        for (int q = 0; q < CPT; ++q) {
-          const double a = ((m >> q) & 1) ? 1.0 : -1.0;
-          f1 += a * P[q];
-          f3 += a * P[q] * P[q] * P[q];
+            for (int q = 0; q < CPT; ++q) {
+              P[q] = c0 + q < ncols ? na[q] + np[q] : 0.0;
+              const double p2 = P[q] * P[q];
+              P3[q] = p2 * P[q];
+              s2 += p2;
+              s4 += p2 * p2;
+            }
+            fetch(cell + 1);
+          }
+          double v[4] = {s2, s4, 0.0, 0.0};
+          signed_sums(__shfl_sync(FULL, my_bits, g + r), v[2], v[3]);
+          const double sum = warp_sum4(v);
+          if (slot == r) mine = sum;
+          if (many >> (g + r) & 1) {
+            // the unit's further copies, two to a reduction, sixteen to an update
+            const uint64_t ph = __shfl_sync(FULL, my_ph, g + r), n = __shfl_sync(FULL, my_n, g + r);
+            for (uint64_t i0 = 1; i0 < n; i0 += 16) {
+              const uint64_t word = lane < 16 && i0 + uint64_t(lane) < n ? copy_bits[ph + i0 + lane] : 0;
+              const uint64_t i = i0 + 2 * slot + (kind >> 1);
+              double* to = i < n ? copy_acc + size_t(ph + i) * 4 + 2 * (kind & 1) : nullptr;
+              const double2 was = to ? *reinterpret_cast<const double2*>(to) : make_double2(0.0, 0.0);
+              double got = 0.0;
+              for (int t = 0; t < 8 && i0 + 2 * t < n; ++t) {
+                double f[4];
+                signed_sums(__shfl_sync(FULL, word, 2 * t), f[0], f[1]);
+                signed_sums(__shfl_sync(FULL, word, 2 * t + 1), f[2], f[3]);
+                const double s = warp_sum4(f);
+                if (slot == t) got = s;
+              }
+              update(to, was, got);
+            }
+          }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          f1 += __shfl_xor_sync(0xffffffffu, f1, o);
-          f3 += __shfl_xor_sync(0xffffffffu, f3, o);
-        }
-        if (uint32_t(lane) == held) {
-          my_copy = ph + i;
-          my_f1 = f1;
-          my_f3 = f3;
-        }
-        if (++held == 32) flush();
+        update(at, old, mine);
       }
     }
-    flush();
   }
 }
 

@@ -42,3 +42,27 @@ def test_copies_across_word_halves(lib, repeats, frequency):
             a, b = np.array(out[block][key]), np.array(out[2][key])
             # the same draws and systems, solved to 1e-12 at another width
             assert np.max(np.abs(a - b)) < 1e-9 * np.max(np.abs(b)), (block, key, a, b)
+
+
+@pytest.mark.parametrize("repeats,frequency", [(7, 1), (9, 2), (1, 16), (2, 17), (1, 18), (3, 34)])
+def test_copies_across_update_groups(lib, repeats, frequency):
+    """Eight rows and sixteen further copies of a row are updated together in the
+    moment pass: counts on both sides of those."""
+    out = {}
+    for block in (2, 8, 64):
+        e = abi.Engine(lib)
+        e.prepare(copies_panel(repeats, frequency), deletion_mode=2)
+        e.device_options(block, 1, 0)
+        q = e.default_request_v5(2)
+        q.v4.v3.v2.algorithm = 2
+        q.v4.v3.engine = 2
+        q.v4.v3.v2.v1.probes = 70
+        q.v4.v3.v2.v1.pcg_tolerance = 1e-12
+        e.solve_v5(q, 4)
+        out[block] = e.result()
+        e.release()
+    for block in (8, 64):
+        for key in ("plugin", "correction", "corrected", "numerical_mcse"):
+            a, b = np.array(out[block][key]), np.array(out[2][key])
+            # the same draws and systems, solved to 1e-12 at another width
+            assert np.max(np.abs(a - b)) < 1e-9 * np.max(np.abs(b)), (block, key, a, b)
