@@ -26,31 +26,33 @@ inline uint32_t warp_chunk(size_t items, int grid) {
 // Cells of a worker are contiguous: [worker_ptr[w], worker_ptr[w+1]).
 // partial[blk][0][K] = |r_W|^2, [1] = |bW|^2.
 template <int K>
-__global__ void k_extract_residual(uint32_t W, uint32_t F, uint32_t chunk, const uint32_t* __restrict__ worker_ptr,
-                                   const uint32_t* __restrict__ cell_firm, const double* __restrict__ cell_weight,
-                                   const double* __restrict__ worker_diag, const int32_t* __restrict__ kept_index,
-                                   const double* __restrict__ x, const double* __restrict__ bW,
-                                   double* __restrict__ alpha, double* __restrict__ partial) {
+__global__ void __launch_bounds__(THREADS) k_extract_residual(
+    uint32_t W, uint32_t F, uint32_t chunk, const uint32_t* __restrict__ worker_ptr,
+    const uint32_t* __restrict__ cell_firm, const double* __restrict__ cell_weight,
+    const double* __restrict__ worker_diag, const int32_t* __restrict__ kept_index, const double* __restrict__ x,
+    const double* __restrict__ bW, double* __restrict__ alpha, double* __restrict__ partial) {
   constexpr int CPT = Cols<K>::CPT, TPR = Cols<K>::TPR;
   double v[2][CPT];
 #pragma unroll
   for (int c = 0; c < CPT; ++c) v[0][c] = v[1][c] = 0.0;
-  auto finish_worker = [&](size_t w, int c0, int32_t k, double d, const double (&acc)[CPT], const double (&b)[CPT]) {
-    const double inv = 1.0 / d;
+  auto finish_worker = [&](size_t w, int c0, int32_t k, double d, double inv, const double (&acc)[CPT]) {
 #pragma unroll
     for (int c = 0; c < CPT; ++c) {
       double al = k >= 0 ? -x[(size_t(F) + k) * K + c0 + c] : acc[c] * inv;
       alpha[w * K + c0 + c] = al;
       double r = acc[c] - d * al;
       v[0][c] += r * r;
-      v[1][c] += b[c] * b[c];
     }
   };
   if constexpr (TPR == 32) {
-    // one warp per `chunk` (at most 32) consecutive workers: their cell ranges, kept indices and
-    // diagonals, and their cells 32 at a time, are loaded lane-parallel and
+    // one warp per `chunk` (at most 32) consecutive workers: their cell ranges,
+    // kept indices and diagonals, and their cells 32 at a time, are loaded lane-parallel and
     // broadcast, so a worker waits only on its own row and its firms' rows;
-    // acc = bW - sum_c w_c psi_f(c) in cell order
+    // acc = bW - sum_c w_c psi_f(c) in cell order.  Bound by the rows' latency
+    // times the warps in flight, so registers count: two firms' rows at a time
+    // and 1/d taken per lane (64 registers) 620 us on 2M workers, against 790
+    // with four rows and a division a worker (80) and 960 with the next two
+    // right-hand sides loaded ahead (96)
     const int lane = threadIdx.x & 31, c0 = lane * CPT;
     const size_t nwarps = size_t(gridDim.x) * blockDim.x / 32;
     for (size_t w0 = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32 * chunk; w0 < W; w0 += nwarps * chunk) {
@@ -64,6 +66,7 @@ __global__ void k_extract_residual(uint32_t W, uint32_t F, uint32_t chunk, const
         my_k = kept_index[w0 + lane];
         my_d = worker_diag[w0 + lane];
       }
+      const double my_inv = 1.0 / my_d;
       uint32_t at = __shfl_sync(0xffffffffu, my_b, 0);  // first cell of the loaded chunk
       const uint32_t last = __shfl_sync(0xffffffffu, my_e, nw - 1);
       uint32_t my_f = 0;
@@ -83,10 +86,11 @@ __global__ void k_extract_residual(uint32_t W, uint32_t F, uint32_t chunk, const
         const int32_t k = __shfl_sync(0xffffffffu, my_k, j);
         const double d = __shfl_sync(0xffffffffu, my_d, j);
         const size_t w = w0 + size_t(j);
-        double acc[CPT], bv[CPT];
+        double acc[CPT];
+        load_cols<K, double>(bW, uint32_t(w), c0, acc);
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) acc[c] = bv[c] = bW[w * K + c0 + c];
-        constexpr int U = 4;
+        for (int c = 0; c < CPT; ++c) v[1][c] += acc[c] * acc[c];
+        constexpr int U = 2;
         for (uint32_t i = b; i < e; i += U) {
           if (i + U > at + 32) load_chunk(i);  // the next items lie past the loaded chunk
           double xv[U][CPT], av[U];
@@ -104,7 +108,7 @@ __global__ void k_extract_residual(uint32_t W, uint32_t F, uint32_t chunk, const
               for (int c = 0; c < CPT; ++c) acc[c] += av[u] * xv[u][c];
             }
         }
-        finish_worker(w, c0, k, d, acc, bv);
+        finish_worker(w, c0, k, d, __shfl_sync(0xffffffffu, my_inv, j), acc);
       }
     }
   } else {
@@ -114,16 +118,19 @@ __global__ void k_extract_residual(uint32_t W, uint32_t F, uint32_t chunk, const
       if (t < total) {
         size_t w = t / TPR;
         int c0 = int(t % TPR) * CPT;
-        double acc[CPT], b[CPT];
+        double acc[CPT];
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) acc[c] = b[c] = bW[w * K + c0 + c];
+        for (int c = 0; c < CPT; ++c) {
+          acc[c] = bW[w * K + c0 + c];
+          v[1][c] += acc[c] * acc[c];
+        }
         for (uint32_t i = worker_ptr[w]; i < worker_ptr[w + 1]; ++i) {
           double a = cell_weight[i];
           size_t fb = size_t(cell_firm[i]) * K + c0;
 #pragma unroll
           for (int c = 0; c < CPT; ++c) acc[c] -= a * x[fb + c];
         }
-        finish_worker(w, c0, kept_index[w], worker_diag[w], acc, b);
+        finish_worker(w, c0, kept_index[w], worker_diag[w], 1.0 / worker_diag[w], acc);
       }
     }
   }
