@@ -48,44 +48,46 @@ namespace fevcb {
 // kernels that are not templated
 
 // out[o] = sum over b of partial[b][o] for o < width, summed in a fixed order.
-// Block x handles FINISH_COLS columns with blockDim / FINISH_COLS lanes each:
-// eight loads in flight a lane, the lanes' sums halved pairwise down to eight
-// (5.2 us for 1,184 partials of 128 columns with four loads and 64 sums added
-// by one thread; 3.4 us so).
-constexpr int FINISH_COLS = 16;
+// Block x handles FINISH_COLS columns with FINISH_THREADS / FINISH_COLS lanes
+// each: ten loads in flight a lane (one round trip for the largest streaming
+// grid), then the lanes of a warp and the warps by shuffles with one block
+// barrier between.  Bound by that chain of latencies: 3.5 us for 1,184 partials
+// of 128 columns, 3.0 for 370 (16 columns a block with 64 lanes each, halved in
+// shared memory on a barrier a step: 7.0 and 4.2).
+constexpr int FINISH_COLS = 8;
 constexpr int FINISH_THREADS = 1024;
 __global__ void __launch_bounds__(FINISH_THREADS) k_finish(const double* __restrict__ partial, int blocks, int width,
                                                            double* __restrict__ out) {
-  __shared__ double sm[FINISH_THREADS];
+  constexpr int WARPS = FINISH_THREADS / 32, GROUPS = FINISH_THREADS / FINISH_COLS;
+  static_assert(WARPS == 32 && FINISH_COLS <= WARPS, "one lane a warp's sum, one warp a column");
+  __shared__ double sm[WARPS][FINISH_COLS];
   partial += size_t(blockIdx.y) * blocks * width;  // one of several partial arrays, one after another
   out += size_t(blockIdx.y) * width;
-  int groups = FINISH_THREADS / FINISH_COLS;
-  const int o = blockIdx.x * FINISH_COLS + threadIdx.x % FINISH_COLS, g = threadIdx.x / FINISH_COLS;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int o = blockIdx.x * FINISH_COLS + threadIdx.x % FINISH_COLS;
   double acc = 0.0;
   if (o < width) {
-    constexpr int U = 8;
-    for (int b0 = g; b0 < blocks; b0 += U * groups) {
+    constexpr int U = 10;
+    for (int b0 = threadIdx.x / FINISH_COLS; b0 < blocks; b0 += U * GROUPS) {
       double v[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int b = b0 + u * groups;
+        const int b = b0 + u * GROUPS;
         v[u] = b < blocks ? partial[size_t(b) * width + o] : 0.0;
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) acc += v[u];
     }
   }
-  sm[threadIdx.x] = acc;
-  __syncthreads();
-  for (; groups > 8; groups >>= 1) {
-    if (g < groups / 2) sm[threadIdx.x] += sm[threadIdx.x + groups / 2 * FINISH_COLS];
-    __syncthreads();
-  }
-  if (g == 0 && o < width) {
-    double sum = 0.0;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) sum += sm[k * FINISH_COLS + threadIdx.x];
-    out[o] = sum;
+  for (int d = FINISH_COLS; d < 32; d <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
+  if (lane < FINISH_COLS) sm[warp][lane] = acc;
+  __syncthreads();
+  if (warp < FINISH_COLS) {
+    double sum = sm[lane][warp];
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+    if (lane == 0 && blockIdx.x * FINISH_COLS + warp < width) out[blockIdx.x * FINISH_COLS + warp] = sum;
   }
 }
 
