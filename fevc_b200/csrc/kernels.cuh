@@ -26,8 +26,8 @@ __device__ __forceinline__ void store4(double* dst, const double (&v)[4]) {
 //   cell_atoms[c*K + j] = sum over the cell's units (exact integers)
 // ALIGNED (first a multiple of four, K >= 4): a thread holds the four probes of
 // one Philox block and stores them as 16-byte pairs; single stores of a
-// thread's four columns each touched every sector of the warp's span (142 ->
-// 70 us for 280,000 cells, 64 probes).  cell_atoms may be null where every cell
+// thread's four columns each touched every sector of the warp's span (420 ->
+// 220 us for 280,000 cells, 64 probes).  cell_atoms may be null where every cell
 // has one unit: the unit atoms are the cell's.
 template <int K, bool ALIGNED>
 __global__ void k_leverage_atoms(uint32_t cells, const uint32_t* __restrict__ unit_ptr,
