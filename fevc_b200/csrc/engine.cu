@@ -301,7 +301,7 @@ struct DeviceEngine {
   int tune_precision[3] = {0, 0, 0}, tune_preconditioner[3] = {0, 0, 0};
   double tune_ms[3] = {0.0, 0.0, 0.0};
   Segments lap_seg, firm_seg;
-  HubRows firm_hubs;  // firms of many segments, summed by a block each
+  HubRows firm_hubs;  // firms of many segments, summed by a block a piece
   int coop_blocks = 0;
   // blocks of the streaming kernels: eight warps each, one warp for every
   // worker, cell or vertex of the problem, at least two blocks an SM and at
@@ -395,7 +395,7 @@ constexpr int PACK_MAX_K = 128;
 struct BlockWork {
   int K;
   DBuf<double> bW, bF, b, x, r, z, p, q, alpha, cell_val, unit_atoms, dir, tot, seg_buf, fseg_out;
-  DBuf<double> hub_sums;  // the hub firms' sums
+  DBuf<double> hub_sums;  // the hub firms' pieces' sums
   // what a solve hands back, in one piece so one copy brings it to the host:
   // 8 K doubles of per-column state, 2 K + 4 ints (active, iterations, nactive,
   // breakdown, replacements, the target balance check), 4 K residual sums
@@ -974,7 +974,7 @@ BlockWork& get_work(DeviceEngine& e) {
   w->tot.alloc(size_t(QMAX + 4) * K);
   w->seg_buf.alloc(size_t(e.lap_seg.count) * K);
   w->fseg_out.alloc(size_t(e.firm_seg.count) * K);
-  w->hub_sums.alloc(size_t(std::max<uint32_t>(e.firm_hubs.count, 1)) * K);
+  w->hub_sums.alloc(size_t(std::max<uint32_t>(e.firm_hubs.pieces, 1)) * K);
   w->pack.alloc(pack_size(K));
   double* st = w->st = w->pack.p;
   int* ist = w->ist = reinterpret_cast<int*>(st + 8 * K);
@@ -1458,11 +1458,12 @@ void firm_gather(DeviceEngine& e, BlockWork& w, Launch L, const double* coef, co
                                                   e.firm_cells.p, e.cell_worker.p, coef, src, total, inv_total,
                                                   w.fseg_out.p);
   const HubRows& hub = e.firm_hubs;
-  if (hub.count)
-    k_hub_rows<K><<<hub.count, HUB_THREADS, 0, L.s>>>(hub.row.p, e.firm_seg.row_first.p, w.fseg_out.p, w.hub_sums.p);
+  if (hub.pieces)
+    k_hub_rows<K><<<hub.pieces, HUB_THREADS, 0, L.s>>>(hub.begin.p, hub.end.p, w.fseg_out.p, w.hub_sums.p);
   k_seg_firm_finish<K, MODE><<<L.grid, THREADS, 0, L.s>>>(e.F, e.kept, e.firm_seg.row_first.p, w.fseg_out.p,
-                                                          hub.count ? hub.slot.p : nullptr, w.hub_sums.p, bF, bW,
-                                                          e.kept_worker.p, e.firm_diag.p, psi, out, partial);
+                                                          hub.pieces ? hub.slot.p : nullptr, hub.first.p,
+                                                          w.hub_sums.p, bF, bW, e.kept_worker.p, e.firm_diag.p, psi,
+                                                          out, partial);
   CK_LAUNCH();
 }
 

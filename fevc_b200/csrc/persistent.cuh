@@ -43,42 +43,55 @@ struct Segments {
 constexpr uint32_t HEAVY_SEGMENTS = 8;
 
 // Rows of a segmented CSR with more than PIECE segments (the hub firms of the
-// firm->cell lists): one block sums each of them, so the rows' finish reads one
-// value for them instead of walking thousands of segments on one warp.
+// firm->cell lists): blocks sum them, HUB_PIECE segments at most each, so the
+// rows' finish reads one value a piece for them instead of walking thousands
+// of segments on one warp.  Nearly every hub is one piece.  A firm of most of
+// a labour market is not: one block for 1.8M workers' cells (56,000 segments,
+// 28 MB at 64 columns) took 289 us on its SM, its 55 pieces take 14.
 constexpr uint32_t PIECE = 32;
+constexpr uint32_t HUB_PIECE = 1024;
 
 struct HubRows {
-  uint32_t count = 0;
-  DBuf<uint32_t> row;   // the hub rows
-  DBuf<int32_t> slot;   // per row: its place in `row`, or -1
+  uint32_t pieces = 0;
+  DBuf<uint32_t> begin, end;  // per piece: its segments
+  DBuf<uint32_t> first;       // per hub row: its pieces [first[h], first[h + 1])
+  DBuf<int32_t> slot;         // per row: its hub row, or -1
 };
 
 inline void build_hub_rows(const std::vector<uint32_t>& row_first, HubRows& hub, cudaStream_t s, uint64_t& h2d) {
   const size_t rows = row_first.size() - 1;
-  std::vector<uint32_t> row;
+  std::vector<uint32_t> begin, end, first(1, 0);
   std::vector<int32_t> slot(rows, -1);
-  for (size_t r = 0; r < rows; ++r)
-    if (row_first[r + 1] - row_first[r] > PIECE) {
-      slot[r] = int32_t(row.size());
-      row.push_back(uint32_t(r));
+  for (size_t r = 0; r < rows; ++r) {
+    const uint32_t s0 = row_first[r], s1 = row_first[r + 1];
+    if (s1 - s0 <= PIECE) continue;
+    slot[r] = int32_t(first.size() - 1);
+    for (uint32_t x = s0; x < s1; x += std::min(HUB_PIECE, s1 - x)) {
+      begin.push_back(x);
+      end.push_back(x + std::min(HUB_PIECE, s1 - x));
     }
-  hub.count = uint32_t(row.size());
-  upload(hub.row, row, s, h2d);
+    first.push_back(uint32_t(begin.size()));
+  }
+  hub.pieces = uint32_t(begin.size());
+  upload(hub.begin, begin, s, h2d);
+  upload(hub.end, end, s, h2d);
+  upload(hub.first, first, s, h2d);
   upload(hub.slot, slot, s, h2d);
 }
 
-// top[h] = sum of hub row h's segments (K columns): the block's groups of TPR
+// top[i] = sum of piece i's segments (K columns): the block's groups of TPR
 // lanes take equal consecutive shares, eight loads in flight, and their sums
 // are halved pairwise: a fixed order, so deterministic.  (Two launches of
-// 32-segment pieces and their pieces cost 8 us at every size; this one 3 to 6.)
+// 32-segment pieces and their pieces cost 8 us at 8 columns, 15 at 64; this
+// one 3 and 8 for a full piece.)
 constexpr int HUB_THREADS = 1024;
 template <int K>
-__global__ void __launch_bounds__(HUB_THREADS) k_hub_rows(const uint32_t* __restrict__ rows,
-                                                          const uint32_t* __restrict__ row_first,
+__global__ void __launch_bounds__(HUB_THREADS) k_hub_rows(const uint32_t* __restrict__ begin,
+                                                          const uint32_t* __restrict__ piece_end,
                                                           const double* __restrict__ seg, double* __restrict__ top) {
   constexpr int CPT = Cols<K>::CPT, TPR = Cols<K>::TPR, U = 8;
   __shared__ double sm[HUB_THREADS * CPT];
-  const uint32_t row = rows[blockIdx.x], s0 = row_first[row], s1 = row_first[row + 1];
+  const uint32_t s0 = begin[blockIdx.x], s1 = piece_end[blockIdx.x];
   int groups = HUB_THREADS / TPR;
   const int g = int(threadIdx.x) / TPR, c0 = int(threadIdx.x % TPR) * CPT;
   const uint32_t per = (s1 - s0 + uint32_t(groups) - 1) / uint32_t(groups);
@@ -960,12 +973,14 @@ __global__ void k_seg_firm(uint32_t nseg, const uint32_t* __restrict__ seg_begin
 //   mode 1: hybrid RHS  b[f] = bF[f] - sum; kept rows b[F+k] = -bW[kept_worker[k]];
 //           partial (sum b, sum b^2)
 //   mode 2: residual    r = bF - d_f psi_f - sum;    partial (|r|^2, |bF|^2)
-// Rows with a hub slot (more than PIECE segments) read their sum from top.
+// Rows with a hub slot (more than PIECE segments) sum their pieces (top_first /
+// top) in order, four loads in flight.
 template <int K, int MODE>
 __global__ void k_seg_firm_finish(uint32_t F, uint32_t kept, const uint32_t* __restrict__ row_first,
                                   const double* __restrict__ seg_out, const int32_t* __restrict__ slot,
-                                  const double* __restrict__ top, const double* __restrict__ bF,
-                                  const double* __restrict__ bW, const uint32_t* __restrict__ kept_worker,
+                                  const uint32_t* __restrict__ top_first, const double* __restrict__ top,
+                                  const double* __restrict__ bF, const double* __restrict__ bW,
+                                  const uint32_t* __restrict__ kept_worker,
                                   const double* __restrict__ firm_diag, const double* __restrict__ psi,
                                   double* __restrict__ out, double* __restrict__ partial) {
   constexpr int CPT = Cols<K>::CPT, TPR = Cols<K>::TPR;
@@ -989,8 +1004,19 @@ __global__ void k_seg_firm_finish(uint32_t F, uint32_t kept, const uint32_t* __r
 #pragma unroll
             for (int c = 0; c < CPT; ++c) acc[c] += seg_out[size_t(sg) * K + c0 + c];
         } else {
+          constexpr uint32_t U = 4;
+          const uint32_t last = top_first[h + 1];
+          for (uint32_t i = top_first[h]; i < last; i += U) {
+            double x[U][CPT];
 #pragma unroll
-          for (int c = 0; c < CPT; ++c) acc[c] = top[size_t(h) * K + c0 + c];
+            for (uint32_t u = 0; u < U; ++u)
+#pragma unroll
+              for (int c = 0; c < CPT; ++c) x[u][c] = i + u < last ? top[size_t(i + u) * K + c0 + c] : 0.0;
+#pragma unroll
+            for (uint32_t u = 0; u < U; ++u)
+#pragma unroll
+              for (int c = 0; c < CPT; ++c) acc[c] += x[u][c];
+          }
         }
         if (MODE == 1) {
 #pragma unroll
