@@ -16,10 +16,10 @@
 // grid-wide reductions an iteration, about 9 us of their 17 us on a
 // 1,000-vertex firm graph.  A 64-column solve of about 20 Jacobi iterations,
 // cooperative against this form: 148 vertices 315 / 45 us, 991 332 / 137 us,
-// 1,391 340 / 220 us, 1,988 350 / 310 us.  Rule of use (column_form,
-// engine.cu): at most COL_MAX_VERTICES vertices, beyond which the matrix, read
-// once per column instead of once per block, costs more than the barriers
-// (2,479 vertices 362 / 417 us, 9,929 583 / 1,717 us).
+// 1,391 340 / 220 us, 1,988 350 / 310 us.  Beyond 2,048 vertices the matrix,
+// read once per column instead of once per block, costs more than the barriers
+// (2,479 vertices 362 / 417 us, 9,929 583 / 1,717 us), and below them so do
+// many entries: column_limit.
 //
 // A finished column's active flag is 0, one at the iteration limit 1, one that
 // met a nonpositive curvature 2; the host counts them (no grid-wide counter).
@@ -65,6 +65,34 @@ inline size_t column_smem(uint32_t n, uint32_t nseg, size_t nnz, bool poly, bool
   const size_t all = vec + nnz * (sizeof(double) + sizeof(uint16_t)) + (size_t(nseg) + 1) * sizeof(uint32_t) + 16;
   *mat = all <= COL_SMEM;
   return n > COL_MAX_VERTICES ? 0 : *mat ? all : vec <= COL_SMEM ? vec : 0;
+}
+
+// Rule of use: entries + 16 vertices of the Laplacian, at most this for a block
+// of K columns.  A column's iteration takes 1.5 us, 0.27 us per 1,000 entries
+// and 3 us per 1,000 vertices on its SM, whatever K; a cooperative iteration is
+// mostly barriers, moves little with the entries and has a dearer start (more
+// of it in a dense graph's few iterations: the vertices' weight).  Solves of
+// panels with 12 to 1,000 workers a firm, cooperative / this form in us, each
+// line's entries on both sides of its limit (thousands):
+//   K = 1      104 321 / 295 (1,000 vertices), 103 345 / 379 (1,900)
+//   K = 2      61 255 / 209 (1,000),           84 292 / 346 (1,500)
+//   K = 8      35 224 / 180 (1,000),           46 245 / 278 (1,500)
+//   K = 16     29 308 / 299 (1,839),           61 187 / 229 (1,000)
+//   K = 32     20 214 / 146 (997),             23 247 / 258 (1,449)   FP64 Jacobi
+//              35 226 / 192 (1,000),           46 258 / 293 (1,500)   k_pcg_flex
+//   K = 64     46 294 / 281 (1,500),           56 298 / 332 (1,897)   FP64 Jacobi
+//              61 320 / 250 (1,000),           56 316 / 350 (1,897)   k_pcg_flex
+// A graph of 1,900 firms and 326,000 entries is where it costs most to miss:
+// 296 / 862 us at K = 64, 216 / 858 at K = 8.
+constexpr size_t column_limit(int K, bool flex) {
+  return K == 1 ? 125000 : K == 2 ? 90000 : K <= 16 ? 62000 : K == 32 ? (flex ? 62000 : 46000) : 80000;
+}
+
+// Whether the column form takes a block of K columns; flex: the cooperative
+// alternative is k_pcg_flex (flex.cuh), poly: the degree-1 stage.
+inline bool column_rule(int K, uint32_t n, uint32_t nseg, size_t nnz, bool flex, bool poly) {
+  bool mat;
+  return nnz + 16 * size_t(n) <= column_limit(K, flex) && column_smem(n, nseg, nnz, poly, &mat) > 0;
 }
 
 inline int column_threads(uint32_t n) { return n <= 64 ? 256 : n <= 256 ? 512 : COL_MAX_THREADS; }

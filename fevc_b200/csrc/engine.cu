@@ -1468,17 +1468,17 @@ void firm_gather(DeviceEngine& e, BlockWork& w, Launch L, const double* coef, co
 }
 
 // The one-block-per-column solve (columns.cuh) serves the Jacobi and the
-// degree-1 forms of Laplacians with at most COL_MAX_VERTICES vertices; as in
-// the cooperative kernels the degree-1 stage takes blocks of 32 or 64 columns.
+// degree-1 forms of small Laplacians (column_rule); as in the cooperative
+// kernels the degree-1 stage takes blocks of 32 or 64 columns.
 template <int K>
 bool column_poly(const DeviceEngine& e) {
   return flex_width<K>() && (e.preconditioner == 3 || e.preconditioner == 4);
 }
 
 template <int K>
-bool column_form(const DeviceEngine& e) {
-  bool mat;
-  return e.preconditioner != 2 && column_smem(e.n, e.lap_seg.count, e.L_col.n, column_poly<K>(e), &mat) > 0;
+bool column_form(const DeviceEngine& e, const SolveOptions& o) {
+  return e.preconditioner != 2 && column_rule(K, e.n, e.lap_seg.count, e.L_col.n, flex_width<K>() && flex_form(e, o),
+                                              column_poly<K>(e));
 }
 
 template <int K>
@@ -1519,7 +1519,7 @@ BlockOutcome solve_block(DeviceEngine& e, BlockWork& w, int ncols, const SolveOp
   BlockOutcome out;
   // hybrid RHS (Schur reduction of the worker block) and its column sums
   firm_gather<K, 1, 1>(e, w, L, e.cell_scale.p, w.bW.p, nullptr, 0.0, w.bF.p, w.bW.p, nullptr, w.b.p, e.partial.p);
-  const bool columns = column_form<K>(e);
+  const bool columns = column_form<K>(e, o);
   if (!columns) {  // (the column solve forms its own means and tolerances)
     finish(e.partial.p, L.grid, 2 * K, w.tot.p, L.s);
     k_pcg_init_state<K><<<1, 128, 0, L.s>>>(w.tot.p, ncols, o.pcg_tolerance, double(e.n), w.s);
