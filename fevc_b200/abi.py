@@ -979,7 +979,9 @@ class Engine:
         3 the learned per-vertex degree-1 stage, 4 the same stage with uniform
         weights) and precision (1: single-precision residual, direction and
         products with a double solution, double reductions and residual
-        replacement)."""
+        replacement; 2: the fastest form of the first leverage block).  Jacobi
+        and degree-1 solves of a small firm graph (at most 2,048 vertices and
+        few entries) hold everything in double for each precision."""
         o = FevcbSolveOptionsV2(FevcbSolveOptionsV1(C.sizeof(FevcbSolveOptionsV2), block_columns, preconditioner, 1),
                                 precision, 0)
         self.check(self.lib.fevcb_engine_solve_options_v1(self.generation, C.byref(o)))

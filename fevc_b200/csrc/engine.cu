@@ -1765,9 +1765,11 @@ void leverage_rhs(DeviceEngine& e, BlockWork& w, Launch L, PhiloxKey key, uint32
 // the FP32 degree-1 stage (learned weights when the engine was built with
 // preconditioner 3, uniform with 4) in the single-kernel PCG.  Every form
 // meets the same FP64 tolerance, so only time decides; the fastest serves
-// every later block and resolve of the generation.  The timing solves are
-// extra work of the first solve only.  With keep_block, a winning last
-// candidate leaves its solve of the first leverage block in the block
+// every later block and resolve of the generation.  A small Laplacian's column
+// solve stores FP64 for every precision, so a candidate that would run an
+// earlier one's kernel takes its time and is not solved again.  The timing
+// solves are extra work of the first solve only.  With tm, a winning candidate
+// that ran last leaves its solve of the first leverage block in the block
 // workspace (right-hand sides, atoms' sign words and solution, exactly what
 // the leverage loop would recompute) for the loop to take over, its counts
 // added to tm.
@@ -1793,14 +1795,24 @@ void autotune(DeviceEngine& e, SolveOptions& o, SolveTimings* tm = nullptr) {
       BlockWork& w = get_work<K>(e);
       Launch L{e.grid, e.stream};
       const PhiloxKey key = philox_key(o.seed);
-      int best = 0;
+      int best = 0, ran = 0;
+      bool column[3];
       SolveTimings scratch;
       BlockOutcome last;
       for (int c = 0; c < nc; ++c) {
-        leverage_rhs<K>(e, w, L, key, 0, K);
         SolveOptions oc = o;
         oc.precision = e.tune_precision[c];
         e.preconditioner = e.tune_preconditioner[c];
+        column[c] = column_form<K>(e, oc);
+        int same = c;
+        for (int d = 0; d < c; ++d)
+          if (column[c] && column[d] && e.tune_preconditioner[c] == e.tune_preconditioner[d]) same = d;
+        if (same != c) {
+          e.tune_ms[c] = e.tune_ms[same];
+          continue;
+        }
+        ran = c;
+        leverage_rhs<K>(e, w, L, key, 0, K);
         scratch = SolveTimings{};
         CK(cudaEventRecord(e.ev0, L.s));
         last = solve_block<K>(e, w, K, oc, scratch);
@@ -1812,7 +1824,7 @@ void autotune(DeviceEngine& e, SolveOptions& o, SolveTimings* tm = nullptr) {
         if (e.tune_ms[c] < e.tune_ms[best]) best = c;
       }
       e.tuned = best;
-      if (tm && best == nc - 1 && o.probe_begin == 0) {
+      if (tm && best == ran && o.probe_begin == 0) {
         e.tuned_block = std::move(last);
         e.tuned_block_width = K;
         tm->pcg_iterations += scratch.pcg_iterations;

@@ -710,7 +710,8 @@ typedef struct FevcbSolveOptionsV2 {
   uint32_t precision;       /* 0 double; 1 single-precision residual, direction and products with a double
                                solution, double reductions and double residual replacement; 2 autotuned:
                                the fastest of those forms on the generation's first leverage block
-                               (fevcb_engine_tuning_v1) */
+                               (fevcb_engine_tuning_v1).  Jacobi and degree-1 solves of a small firm graph (at
+                               most 2,048 vertices and few entries) hold everything in double for each value */
   uint32_t reserved;
 } FevcbSolveOptionsV2;
 
@@ -888,7 +889,9 @@ int32_t fevcb_engine_kernel_benchmark_v1(uint64_t generation, uint32_t kernel, u
  * counterpart in the reference): the candidates timed on the first leverage
  * block (precision 0/1 and preconditioner 1 Jacobi, 3 learned or 4 uniform
  * degree-1 stage), their milliseconds, and the index of the one kept
- * (-1 before the first such solve). */
+ * (-1 before the first such solve).  On a small firm graph precision 0 and 1
+ * are one solve in double: the Jacobi candidates then have one time, and the
+ * first of them stands for both. */
 typedef struct FevcbTuningV1 {
   uint32_t struct_size;
   int32_t chosen;
