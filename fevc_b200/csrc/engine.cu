@@ -1350,8 +1350,10 @@ void mg_iteration(DeviceEngine& e, BlockWork& w, Launch L, cudaStream_t s) {
 
 constexpr int MG_GRAPH_ITERATIONS = 4;
 
+// `balance` (solve_block) is called with its word at the first state read.
 template <int K>
-int pcg_run_mg(DeviceEngine& e, BlockWork& w, Launch L, int iterations, SolveTimings& tm) {
+int pcg_run_mg(DeviceEngine& e, BlockWork& w, Launch L, int iterations, SolveTimings& tm,
+               const std::function<void(int)>* balance = nullptr) {
   if (!w.graph) {
     cudaGraph_t g = nullptr;
     // launches recorded into the graph run only when it is replayed: take
@@ -1370,7 +1372,9 @@ int pcg_run_mg(DeviceEngine& e, BlockWork& w, Launch L, int iterations, SolveTim
   }
   int executed = 0;
   CK(cudaMemcpyAsync(e.h_nactive, w.s.nactive, sizeof(int), cudaMemcpyDeviceToHost, L.s));
+  if (balance) CK(cudaMemcpyAsync(e.h_nactive + 2, w.ist + 2 * K + 3, sizeof(int), cudaMemcpyDeviceToHost, L.s));
   CK(cudaStreamSynchronize(L.s));
+  if (balance) (*balance)(e.h_nactive[2]);
   while (*e.h_nactive > 0 && executed < iterations) {
     CK(cudaGraphLaunch(w.graph, L.s));
     executed += w.graph_iters;
@@ -1437,11 +1441,14 @@ int run_fallback(DeviceEngine& e, BlockWork& w, Launch L, int budget, int used, 
 // state comes back with the extraction results), else runs the CMG fallback
 // and returns its largest per-column iteration count.
 template <int K>
-int learned_fallback(DeviceEngine& e, BlockWork& w, Launch L, int budget, SolveTimings& tm) {
+int learned_fallback(DeviceEngine& e, BlockWork& w, Launch L, int budget, SolveTimings& tm,
+                     const std::function<void(int)>* balance) {
   int bd = -1;
   CK(cudaMemcpyAsync(e.h_nactive, w.s.nactive, sizeof(int), cudaMemcpyDeviceToHost, L.s));
   CK(cudaMemcpyAsync(&bd, w.s.breakdown, sizeof(int), cudaMemcpyDeviceToHost, L.s));
+  if (balance) CK(cudaMemcpyAsync(e.h_nactive + 2, w.ist + 2 * K + 3, sizeof(int), cudaMemcpyDeviceToHost, L.s));
   CK(cudaStreamSynchronize(L.s));
+  if (balance) (*balance)(e.h_nactive[2]);
   if (*e.h_nactive == 0 && bd < 0) return -1;
   std::vector<int> it(K);
   CK(cudaMemcpyAsync(it.data(), w.s.iters, K * sizeof(int), cudaMemcpyDeviceToHost, L.s));
@@ -1511,7 +1518,8 @@ void launch_columns(DeviceEngine& e, BlockWork& w, Launch L, int ncols, double t
 // On return w.alpha holds the worker solution and w.x[0, F) the firm solution.
 // One host round trip: the state, the residual sums and the flags come back in
 // one pinned copy after the extraction.  balance: called with the target
-// balance check's word (k_balance_repair) before the solve's own checks.
+// balance check's word (k_balance_repair) at the first round trip, before the
+// solve's own checks.
 template <int K>
 BlockOutcome solve_block(DeviceEngine& e, BlockWork& w, int ncols, const SolveOptions& o, SolveTimings& tm,
                          const std::function<void(int)>* balance = nullptr) {
@@ -1557,9 +1565,9 @@ BlockOutcome solve_block(DeviceEngine& e, BlockWork& w, int ncols, const SolveOp
       const bool learned = e.preconditioner == 3;
       launch_flex<K>(e, w, L, learned ? std::min(budget, LEARNED_CAP) : budget, ladder == 0, o.precision);
       tm.spmm_launches += 1;
-      done = learned ? learned_fallback<K>(e, w, L, budget, tm) : -1;
+      done = learned ? learned_fallback<K>(e, w, L, budget, tm, balance) : -1;
     } else if (e.preconditioner == 2) {
-      done = pcg_run_mg<K>(e, w, L, budget, tm);
+      done = pcg_run_mg<K>(e, w, L, budget, tm, balance);
     } else {
       // the Jacobi kernel's active count and iterations come back with the
       // extraction results below (no host round trip of its own)
@@ -1896,6 +1904,7 @@ void run_target(DeviceEngine& e, const SolveOptions& o, SolveResult& res, double
   SmallMatrix sinv{};
   for (int k = 0; k < e.qa; ++k)
     for (int l = 0; l < e.qa; ++l) sinv.m[k * QMAX + l] = e.Sinv[k * e.qa + l];
+  std::exception_ptr failed;
   for (uint32_t first = o.probe_begin; first < end; first += H) {
     int np = int(std::min<uint32_t>(H, end - first));
     double* sums = e.draw_sums.p + outcomes.size() * slot;
@@ -1930,7 +1939,12 @@ void run_target(DeviceEngine& e, const SolveOptions& o, SolveResult& res, double
       fail(TARGET_CENTERING_FAILED, "jla_target",
            "compatibility repair exceeded roundoff at probe " + probe + ((q & 1) ? ", side Firm" : ", side Worker"));
     };
-    outcomes.push_back(solve_block<K>(e, w, 2 * np, o, res.timings, &balance));
+    try {
+      outcomes.push_back(solve_block<K>(e, w, 2 * np, o, res.timings, &balance));
+    } catch (...) {
+      failed = std::current_exception();
+      break;
+    }
     if (!e.generic) {
       if (o.numerical)  // the contraction plus the cells' target fold sums of the attachment
         k_contract_folds<K><<<L.grid, THREADS, 0, L.s>>>(e.C, e.cell_worker.p, e.cell_firm.p, e.omega.p, w.alpha.p,
@@ -1985,7 +1999,8 @@ void run_target(DeviceEngine& e, const SolveOptions& o, SolveResult& res, double
     }
     CK_LAUNCH();
   }
-  // the draws of every block
+  // the draws of every solved block; a nonfinite draw is reported ahead of a
+  // later block's failure
   std::vector<double> all(slot * outcomes.size()), beta(QMAX * K, 0.0), draws(3 * K), g2(2 * K);
   if (!all.empty())
     CK(cudaMemcpyAsync(all.data(), e.draw_sums.p, all.size() * sizeof(double), cudaMemcpyDeviceToHost, L.s));
@@ -2059,6 +2074,7 @@ void run_target(DeviceEngine& e, const SolveOptions& o, SolveResult& res, double
                                         uint32_t(bo.zero[2 * j + 1]), bo.reduced[2 * j + 1], bo.complete[2 * j + 1]});
     }
   }
+  if (failed) std::rethrow_exception(failed);
 }
 
 // Probe blocks: full blocks at width K, and a last partial block at the
