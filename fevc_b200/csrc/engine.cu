@@ -1468,9 +1468,8 @@ void firm_gather(DeviceEngine& e, BlockWork& w, Launch L, const double* coef, co
   if (hub.pieces)
     k_hub_rows<K><<<hub.pieces, HUB_THREADS, 0, L.s>>>(hub.begin.p, hub.end.p, w.fseg_out.p, w.hub_sums.p);
   k_seg_firm_finish<K, MODE><<<L.grid, THREADS, 0, L.s>>>(e.F, e.kept, e.firm_seg.row_first.p, w.fseg_out.p,
-                                                          hub.pieces ? hub.slot.p : nullptr, hub.first.p,
-                                                          w.hub_sums.p, bF, bW, e.kept_worker.p, e.firm_diag.p, psi,
-                                                          out, partial);
+                                                          hub.pieces ? hub.slot.p : nullptr, w.hub_sums.p, bF, bW,
+                                                          e.kept_worker.p, e.firm_diag.p, psi, out, partial);
   CK_LAUNCH();
 }
 

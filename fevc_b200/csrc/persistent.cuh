@@ -54,28 +54,26 @@ constexpr uint32_t HUB_PIECE = 1024;
 struct HubRows {
   uint32_t pieces = 0;
   DBuf<uint32_t> begin, end;  // per piece: its segments
-  DBuf<uint32_t> first;       // per hub row: its pieces [first[h], first[h + 1])
-  DBuf<int32_t> slot;         // per row: its hub row, or -1
+  DBuf<uint2> slot;           // per row: its pieces [x, y), none for x = y
 };
 
 inline void build_hub_rows(const std::vector<uint32_t>& row_first, HubRows& hub, cudaStream_t s, uint64_t& h2d) {
   const size_t rows = row_first.size() - 1;
-  std::vector<uint32_t> begin, end, first(1, 0);
-  std::vector<int32_t> slot(rows, -1);
+  std::vector<uint32_t> begin, end;
+  std::vector<uint2> slot(rows, make_uint2(0, 0));
   for (size_t r = 0; r < rows; ++r) {
     const uint32_t s0 = row_first[r], s1 = row_first[r + 1];
     if (s1 - s0 <= PIECE) continue;
-    slot[r] = int32_t(first.size() - 1);
+    slot[r].x = uint32_t(begin.size());
     for (uint32_t x = s0; x < s1; x += std::min(HUB_PIECE, s1 - x)) {
       begin.push_back(x);
       end.push_back(x + std::min(HUB_PIECE, s1 - x));
     }
-    first.push_back(uint32_t(begin.size()));
+    slot[r].y = uint32_t(begin.size());
   }
   hub.pieces = uint32_t(begin.size());
   upload(hub.begin, begin, s, h2d);
   upload(hub.end, end, s, h2d);
-  upload(hub.first, first, s, h2d);
   upload(hub.slot, slot, s, h2d);
 }
 
@@ -973,14 +971,13 @@ __global__ void k_seg_firm(uint32_t nseg, const uint32_t* __restrict__ seg_begin
 //   mode 1: hybrid RHS  b[f] = bF[f] - sum; kept rows b[F+k] = -bW[kept_worker[k]];
 //           partial (sum b, sum b^2)
 //   mode 2: residual    r = bF - d_f psi_f - sum;    partial (|r|^2, |bF|^2)
-// Rows with a hub slot (more than PIECE segments) sum their pieces (top_first /
-// top) in order, four loads in flight.
+// Rows with pieces (more than PIECE segments) sum those in order, four loads in
+// flight.
 template <int K, int MODE>
 __global__ void k_seg_firm_finish(uint32_t F, uint32_t kept, const uint32_t* __restrict__ row_first,
-                                  const double* __restrict__ seg_out, const int32_t* __restrict__ slot,
-                                  const uint32_t* __restrict__ top_first, const double* __restrict__ top,
-                                  const double* __restrict__ bF, const double* __restrict__ bW,
-                                  const uint32_t* __restrict__ kept_worker,
+                                  const double* __restrict__ seg_out, const uint2* __restrict__ slot,
+                                  const double* __restrict__ top, const double* __restrict__ bF,
+                                  const double* __restrict__ bW, const uint32_t* __restrict__ kept_worker,
                                   const double* __restrict__ firm_diag, const double* __restrict__ psi,
                                   double* __restrict__ out, double* __restrict__ partial) {
   constexpr int CPT = Cols<K>::CPT, TPR = Cols<K>::TPR;
@@ -998,20 +995,19 @@ __global__ void k_seg_firm_finish(uint32_t F, uint32_t kept, const uint32_t* __r
       if (f < F) {
 #pragma unroll
         for (int c = 0; c < CPT; ++c) acc[c] = 0.0;
-        const int32_t h = slot ? slot[f] : -1;
-        if (h < 0) {
+        const uint2 h = slot ? slot[f] : make_uint2(0, 0);
+        if (h.x == h.y) {
           for (uint32_t sg = row_first[f]; sg < row_first[f + 1]; ++sg)
 #pragma unroll
             for (int c = 0; c < CPT; ++c) acc[c] += seg_out[size_t(sg) * K + c0 + c];
         } else {
           constexpr uint32_t U = 4;
-          const uint32_t last = top_first[h + 1];
-          for (uint32_t i = top_first[h]; i < last; i += U) {
+          for (uint32_t i = h.x; i < h.y; i += U) {
             double x[U][CPT];
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u)
 #pragma unroll
-              for (int c = 0; c < CPT; ++c) x[u][c] = i + u < last ? top[size_t(i + u) * K + c0 + c] : 0.0;
+              for (int c = 0; c < CPT; ++c) x[u][c] = i + u < h.y ? top[size_t(i + u) * K + c0 + c] : 0.0;
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u)
 #pragma unroll
