@@ -1350,7 +1350,16 @@ void mg_iteration(DeviceEngine& e, BlockWork& w, Launch L, cudaStream_t s) {
 
 constexpr int MG_GRAPH_ITERATIONS = 4;
 
-// `balance` (solve_block) is called with its word at the first state read.
+// Read the flags of a block's state (active columns, breakdown, replacements,
+// the target balance check's word) into h_nactive[0..3] in one copy; `balance`
+// (solve_block) is called with its word.
+template <int K>
+void read_flags(DeviceEngine& e, BlockWork& w, Launch L, const std::function<void(int)>* balance) {
+  CK(cudaMemcpyAsync(e.h_nactive, w.ist + 2 * K, 4 * sizeof(int), cudaMemcpyDeviceToHost, L.s));
+  CK(cudaStreamSynchronize(L.s));
+  if (balance) (*balance)(e.h_nactive[3]);
+}
+
 template <int K>
 int pcg_run_mg(DeviceEngine& e, BlockWork& w, Launch L, int iterations, SolveTimings& tm,
                const std::function<void(int)>* balance = nullptr) {
@@ -1371,10 +1380,7 @@ int pcg_run_mg(DeviceEngine& e, BlockWork& w, Launch L, int iterations, SolveTim
     w.graph_iters = MG_GRAPH_ITERATIONS;
   }
   int executed = 0;
-  CK(cudaMemcpyAsync(e.h_nactive, w.s.nactive, sizeof(int), cudaMemcpyDeviceToHost, L.s));
-  if (balance) CK(cudaMemcpyAsync(e.h_nactive + 2, w.ist + 2 * K + 3, sizeof(int), cudaMemcpyDeviceToHost, L.s));
-  CK(cudaStreamSynchronize(L.s));
-  if (balance) (*balance)(e.h_nactive[2]);
+  read_flags<K>(e, w, L, balance);
   while (*e.h_nactive > 0 && executed < iterations) {
     CK(cudaGraphLaunch(w.graph, L.s));
     executed += w.graph_iters;
@@ -1443,13 +1449,8 @@ int run_fallback(DeviceEngine& e, BlockWork& w, Launch L, int budget, int used, 
 template <int K>
 int learned_fallback(DeviceEngine& e, BlockWork& w, Launch L, int budget, SolveTimings& tm,
                      const std::function<void(int)>* balance) {
-  int bd = -1;
-  CK(cudaMemcpyAsync(e.h_nactive, w.s.nactive, sizeof(int), cudaMemcpyDeviceToHost, L.s));
-  CK(cudaMemcpyAsync(&bd, w.s.breakdown, sizeof(int), cudaMemcpyDeviceToHost, L.s));
-  if (balance) CK(cudaMemcpyAsync(e.h_nactive + 2, w.ist + 2 * K + 3, sizeof(int), cudaMemcpyDeviceToHost, L.s));
-  CK(cudaStreamSynchronize(L.s));
-  if (balance) (*balance)(e.h_nactive[2]);
-  if (*e.h_nactive == 0 && bd < 0) return -1;
+  read_flags<K>(e, w, L, balance);
+  if (e.h_nactive[0] == 0 && e.h_nactive[1] < 0) return -1;
   std::vector<int> it(K);
   CK(cudaMemcpyAsync(it.data(), w.s.iters, K * sizeof(int), cudaMemcpyDeviceToHost, L.s));
   CK(cudaStreamSynchronize(L.s));
