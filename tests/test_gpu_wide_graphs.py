@@ -59,3 +59,24 @@ def test_cooperative_forms_match_the_oracle(lib, tmp_path, want, block, precondi
     for key, okey in (("plugin", "plugin"), ("corrected", "corrected"), ("numerical_mcse", "mcse")):
         a, b = np.array(got[key]), want[okey]
         assert np.max(np.abs(a - b)) < 1e-8 * np.max(np.abs(b)), key  # the suite's component tolerance
+
+
+@pytest.mark.parametrize("preconditioner,precision", [(1, 1), (4, 0), (3, 1)])
+def test_exact_leverages_agree_between_the_forms(lib, preconditioner, precision):
+    """The exact estimator above the column solve's size: every form's blocks
+    give the FP64 Jacobi form's components."""
+    if preconditioner == 3:
+        learned.install(lib, learned.load_params())
+    out = []
+    for pre, prec in ((1, 0), (preconditioner, precision)):
+        e = abi.Engine(lib)
+        e.prepare(generate_panel(6_000, 2_600, 6, move_p=0.3, pareto_shape=2.5, seed=1))
+        e.device_options(64, pre, prec)
+        e.exact_ceiling(1_000_000)
+        e.solve_v5(e.exact_request_v5())
+        assert e.timings()["vertices"] > 2048
+        out.append(e.result())
+        e.release()
+    for key in ("plugin", "correction", "corrected"):
+        a, b = np.array(out[1][key]), np.array(out[0][key])
+        assert np.max(np.abs(a - b)) < 1e-8 * np.max(np.abs(b)), key  # the suite's component tolerance
