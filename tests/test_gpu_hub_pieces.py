@@ -5,7 +5,7 @@ and segments, and many pieces, at every kind of block width."""
 import numpy as np
 import pytest
 
-from device_trace import kernels
+from device_trace import resolve_kernels
 from fevc_b200 import abi
 from fevc_b200.panel import Panel
 from oracle import oracle
@@ -41,7 +41,7 @@ def test_hub_pieces_match_the_oracle(lib, tmp_path, cells, block):
     q.pcg_tolerance = 1e-12
     e.solve(q)
     got = e.result()
-    launched = kernels(e.resolve, tmp_path)
+    launched = resolve_kernels(e, tmp_path)
     want = oracle.run(oracle.problem_view(lib, e.generation), probes=probes)
     e.release()
     for key, okey in (("plugin", "plugin"), ("corrected", "corrected"), ("numerical_mcse", "mcse")):

@@ -5,7 +5,7 @@ multigrid form, the iteration limit and a nonpositive curvature."""
 import numpy as np
 import pytest
 
-from device_trace import count, kernels
+from device_trace import count, resolve_kernels
 from fevc_b200 import abi, learned
 from fevc_b200.panel import Panel, generate_panel
 
@@ -54,7 +54,7 @@ def test_capped_learned_solve_falls_back_to_multigrid(lib, tmp_path, firms, kern
     panel = ring_panel(firms)
     e = solve(lib, panel, block, 3, precision, probes)
     got, t, receipts = e.result(), e.timings(), e.rhs_receipts(1 + 3 * probes)
-    launched = kernels(e.resolve, tmp_path)
+    launched = resolve_kernels(e, tmp_path)
     again, t2 = e.result(), e.timings()
     e.release()
     assert t["vertices"] == firms

@@ -5,7 +5,7 @@ dense graphs, and the same components either way."""
 import numpy as np
 import pytest
 
-from device_trace import count, kernels
+from device_trace import count, resolve_kernels
 from fevc_b200 import abi
 from fevc_b200.panel import generate_panel
 
@@ -29,7 +29,7 @@ def run(lib, tmp_path, spec, block, preconditioner, precision, probes):
     q.v4.v3.v2.v1.pcg_tolerance = 1e-12
     e.solve_v5(q)
     res, t = e.result(), e.timings()
-    launched = kernels(e.resolve, tmp_path)
+    launched = resolve_kernels(e, tmp_path)
     e.release()
     return res, t, launched
 

@@ -4,7 +4,7 @@ a dense one every candidate is solved."""
 
 import pytest
 
-from device_trace import kernels
+from device_trace import kernels, resolve_kernels
 from fevc_b200 import abi
 from fevc_b200.panel import generate_panel
 
@@ -19,14 +19,14 @@ def run(lib, tmp_path, spec, preconditioner, precision):
     q = e.default_request()
     q.probes = 64
 
-    def solves(call):
+    def solves(launched):
         wide = ("k_pcg_flex<64", "k_pcg_persistent<64")
         return sum(name.startswith(wide) or (name.startswith("k_pcg_columns") and grid[0] == 64)
-                   for name, grid, _ in kernels(call, tmp_path))
+                   for name, grid, _ in launched)
 
-    first = solves(lambda: e.solve(q))
+    first = solves(kernels(lambda: e.solve(q), tmp_path))
     res, tuning = e.result(), e.tuning()
-    assert solves(e.resolve) == 3  # one leverage block, two target blocks
+    assert solves(resolve_kernels(e, tmp_path)) == 3  # one leverage block, two target blocks
     assert e.result() == res
     e.release()
     return res, tuning, first

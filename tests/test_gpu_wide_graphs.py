@@ -4,7 +4,7 @@
 import numpy as np
 import pytest
 
-from device_trace import kernels
+from device_trace import resolve_kernels
 from fevc_b200 import abi, learned
 from fevc_b200.panel import generate_panel
 from oracle import oracle
@@ -50,7 +50,7 @@ def test_cooperative_forms_match_the_oracle(lib, tmp_path, want, block, precondi
     e.solve(q)
     got, t = e.result(), e.timings()
     receipts = e.rhs_receipts(1 + 3 * PROBES)
-    names = [name for name, _, _ in kernels(e.resolve, tmp_path)]
+    names = [name for name, _, _ in resolve_kernels(e, tmp_path)]
     e.release()
     assert t["vertices"] > 2048 and t["fallbacks"] == 0
     assert any(name.startswith(kernel) for name in names), sorted(set(names))
